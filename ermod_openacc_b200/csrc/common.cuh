@@ -67,7 +67,8 @@ __device__ __forceinline__ float pair_energy(const PairParams& P, float dis2, fl
   const float rinv = __frsqrt_rn(dis2);
   const float rst = dis2 > 0.0f ? dis2 * rinv : 0.0f;   // coincident sites: r = 0, as sqrt gives
   float eplj = 0.0f;
-  if (!(rst > P.up)) {
+  // a zero epsilon (a water hydrogen) gives a zero term, except where r^-12 overflows
+  if (!(rst > P.up) && !(ljeps == 0.0f && dis2 > 1.0e-2f)) {
     const float invr2 = ljsgm2 * (rinv * rinv);
     const float invr6 = invr2 * invr2 * invr2;
     if (P.ljswitch <= 1) {

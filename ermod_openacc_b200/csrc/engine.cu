@@ -66,7 +66,6 @@ struct ermod_ctx {
   std::vector<int> uvmax, uvsoft;
   DeviceState d;
   int chunk = kChunk, batch = 0, ncell_cap = 0;
-  float cell_h = 0.f;                    // cell-list edge picked by the tuner (0: not yet tuned, 4 A)
   int nhost = 0;                      // atoms of the host aggregate (insposition 2..4)
   int nref = 0;                       // atoms of the RefInfo host (insposition 5, 6)
   bool gauss_init = false;            // Gaussian insertion constants fixed at the first frame
@@ -131,7 +130,8 @@ void free_all(ermod_ctx* c) {
   DeviceState& d = c->d;
   void* ptrs[] = {d.molbeg, d.molspec, d.molq, d.atom_lj, d.atom_q, d.ljene, d.ljlensq, d.slt_lj, d.slt_q,
                   d.slt_mass, d.bfcoord, d.uvcrd, d.spec_off, d.uvsoft, d.escrd, d.posraw, d.slvn, d.spl, d.grd,
-                  d.grec, d.mrec, d.anchor, d.cellof, d.cellcount, d.cellstart, d.molsorted, d.rmol, d.ins_conf, d.insw_in,
+                  d.grec, d.mrec, d.sanch, d.gsph, d.anchor, d.cellof, d.cellcount, d.cellstart, d.molsorted, d.ins_conf,
+                  d.insw_in,
                   d.tgt_raw, d.tgt_n, d.tgt_c, d.tgt_mol, d.selfreal, d.selfrec, d.u0, d.w, d.etot, d.flceng,
                   d.grid, d.spec, d.phin, d.phi, d.engfac, d.engfacT, d.fft_tw, d.fft_twd, d.sitetab, d.sitestn,
                   d.splfc,
@@ -431,9 +431,10 @@ int32_t ermod_create(ermod_ctx** out, int32_t device, const ermod_params* prm, c
   CK(dalloc(&d.uvcrd, ctx->ermax)); CK(dalloc(&d.spec_off, ctx->numslv + 1)); CK(dalloc(&d.uvsoft, ctx->numslv));
   CK(dalloc(&d.escrd, std::max(1, ctx->esmax)));
   CK(dalloc(&d.posraw, 3 * NA)); CK(dalloc(&d.slvn, NA)); CK(dalloc(&d.spl, NA * 3 * order)); CK(dalloc(&d.grd, NA));
-  if (pme && gather_rec_ok(order, K1, K2, K3)) { CK(dalloc(&d.grec, NA * kRecWords)); CK(dalloc(&d.mrec, SM)); }
+  if (pme && gather_rec_ok(order, K1, K2, K3)) CK(dalloc(&d.grec, NA * kRecWords));
+  CK(dalloc(&d.mrec, SM)); CK(dalloc(&d.sanch, SM)); CK(dalloc(&d.gsph, (SM + 31) / 32));
   CK(dalloc(&d.anchor, SM)); CK(dalloc(&d.cellof, SM)); CK(dalloc(&d.cellcount, ctx->ncell_cap));
-  CK(dalloc(&d.cellstart, ctx->ncell_cap + 1)); CK(dalloc(&d.molsorted, SM)); CK(dalloc(&d.rmol, 1));
+  CK(dalloc(&d.cellstart, ctx->ncell_cap + 1)); CK(dalloc(&d.molsorted, SM));
   CK(dalloc(&d.ins_conf, 3 * S * MD)); CK(dalloc(&d.insw_in, MD));
   CK(dalloc(&d.tgt_raw, MD * S)); CK(dalloc(&d.tgt_n, MD * S)); CK(dalloc(&d.tgt_c, MD)); CK(dalloc(&d.tgt_mol, MD));
   CK(dalloc(&d.selfreal, MD)); CK(dalloc(&d.selfrec, MD)); CK(dalloc(&d.u0, MD)); CK(dalloc(&d.w, MD));
@@ -442,7 +443,7 @@ int32_t ermod_create(ermod_ctx** out, int32_t device, const ermod_params* prm, c
   // PME solve path (spectrum_path): the fused solve where the mesh allows it
   FrameArgs fa{};
   fa.pme = pme; fa.K1 = K1; fa.K2 = K2; fa.K3 = K3; fa.Kh1 = Kh1; fa.nsite = ctx->s; fa.order = order;
-  fa.ljtype_max = ctx->ljtype_max;
+  fa.ljtype_max = ctx->ljtype_max; fa.slvmax = ctx->slvmax; fa.maxdst = ctx->maxdst;
   if (setup_real_smem(fa) != 0) return bad(ERMOD_ERR_CUDA, "real_smem");
   if (setup_insert_smem(ctx->s) != 0) return bad(ERMOD_ERR_CUDA, "ins_smem");
   const bool fused_ok = pme && fused_supported(fa);
@@ -691,18 +692,16 @@ struct FramePlanHost {
   double inv[3][3], vold;
 };
 
-// Cell grid of the real-space cell list for cells of edge >= hmin on the normalised cuboid
-// box (at most 64 a side, at least 3); false when no such grid fits.
-constexpr float kCellDefault = 4.0f;
-static bool cell_grid(const ermod_ctx* ctx, FrameArgs& a, float hmin, int& ncell) {
-  bool ok = true;
+// Cells of the molecules' spatial order on the normalised cuboid box, about four molecules each
+// (a block of 2 x 2 x 2 cells is then about one group of 32), at most 64 a side.
+static void cell_grid(const ermod_ctx* ctx, FrameArgs& a, int& ncell) {
+  const float edge = std::cbrt(4.0f * a.g.len[0] * a.g.len[1] * a.g.len[2] / (float)std::max(1, ctx->slvmax));
+  ncell = 8;
   for (int dd = 0; dd < 3; ++dd) {
-    a.nc[dd] = std::max(1, std::min(64, (int)std::floor(a.g.len[dd] / hmin)));
+    a.nc[dd] = std::max(1, std::min(64, (int)std::floor(a.g.len[dd] / edge)));
     a.ch[dd] = a.g.len[dd] / (float)a.nc[dd];
-    if (a.nc[dd] < 3) ok = false;
+    ncell *= (a.nc[dd] + 1) / 2;
   }
-  ncell = a.nc[0] * a.nc[1] * a.nc[2];
-  return ok && ncell <= ctx->ncell_cap;
 }
 
 static int frame_plan(ermod_ctx* ctx, const float* cellin, float wsys, bool use_conf, FramePlanHost& ph) {
@@ -852,11 +851,12 @@ static int frame_plan(ermod_ctx* ctx, const float* cellin, float wsys, bool use_
   a.pivol = pme ? kPi / ((double)p.screen * (double)p.screen) / vold : 0.0;
   a.rcut = g.periodic ? std::max(p.elecut, p.upljcut) : (P.bare ? FLT_MAX : p.upljcut);
   if (P.bare && !g.periodic) a.rcut = FLT_MAX;
-  // cell list only for cuboid periodic boxes
+  // spatial order only for cuboid periodic boxes; other molecules keep their order
   a.use_cells = 0;
   fp.ncell = 1;
   if (g.periodic && g.cuboid && !g.rotated) {
-    a.use_cells = cell_grid(ctx, a, ctx->cell_h > 0.f ? ctx->cell_h : kCellDefault, fp.ncell) ? 1 : 0;
+    cell_grid(ctx, a, fp.ncell);
+    a.use_cells = 1;
   }
   // ---- influence function when the cell changes (engconst :423-433) ----
   if (pme) {
@@ -930,49 +930,31 @@ static void frame_commit(ermod_ctx* ctx, const float* cellin, const FramePlanHos
   if (ph.k.selfreal == 1) ctx->usreal_init = true;
 }
 
-// Block size of k_real: the autotuner's candidates all give bit-identical
-// energies (a warp per molecule whatever the block size), so the choice only
-// moves time.  Tuned on the first frame with the frame's own data.
-static const int kRealCandidates[] = {128, 256, 512};
-static const float kCellCandidates[] = {3.0f, 4.0f, 5.0f, 6.0f};
+// Block size of k_real: the autotuner's candidates all give bit-identical energies (a molecule's
+// sum does not depend on the block it runs in), so the choice only moves time.
+static const int kRealCandidates[] = {64, 128, 256};
 
-// The real-space autotuner, run on the first frame with that frame's own data: every cell
-// edge of kCellCandidates (on cuboid periodic boxes) times every block size of
-// kRealCandidates, each timed on the second of two launches; the fastest pair is kept for
-// the context's later frames.  A molecule's energy is one fixed-order sum whatever the cell
-// grid and block size, so the choice moves only time.  The frame's own cell list is rebuilt
-// afterwards, so the rest of this frame runs on the grid it was planned with.
-static int tune_real(ermod_ctx* ctx, const FrameArgs& a, int ncell0, int nbatch, cudaStream_t st) {
+// The real-space autotuner, run on the first frame with that frame's own data: every block size of
+// kRealCandidates, each timed on the second of two launches; the fastest is kept for the context's
+// later frames.
+static int tune_real(ermod_ctx* ctx, const FrameArgs& a, int nbatch, cudaStream_t st) {
   float best = 1e30f;
-  int pick = 256;
-  float hpick = kCellDefault;
+  int pick = 128;
   cudaEvent_t e0 = ctx->ev[0], e1 = ctx->ev[1];
-  const int nh = a.use_cells ? (int)(sizeof(kCellCandidates) / sizeof(float)) : 1;
-  for (int ih = 0; ih < nh; ++ih) {
-    FrameArgs b = a;
-    if (a.use_cells) {
-      int nc = 0;
-      if (!cell_grid(ctx, b, kCellCandidates[ih], nc)) continue;
-      launch_cells(b, ctx->d, nc, st);
-    }
-    for (int rep = 0; rep < 2; ++rep)
-      for (int nt : kRealCandidates) {
-        CK(cudaEventRecord(e0, st));
-        launch_real(b, ctx->d, 0, nbatch, ctx->batch, nt, st);
-        CK(cudaEventRecord(e1, st));
-        CK(cudaEventSynchronize(e1));
-        float ms = 0.f;
-        CK(cudaEventElapsedTime(&ms, e0, e1));
-        if (rep == 1 && ms < best) {
-          best = ms;
-          pick = nt;
-          hpick = a.use_cells ? kCellCandidates[ih] : kCellDefault;
-        }
+  for (int rep = 0; rep < 2; ++rep)
+    for (int nt : kRealCandidates) {
+      CK(cudaEventRecord(e0, st));
+      launch_real(a, ctx->d, 0, nbatch, ctx->batch, nt, st);
+      CK(cudaEventRecord(e1, st));
+      CK(cudaEventSynchronize(e1));
+      float ms = 0.f;
+      CK(cudaEventElapsedTime(&ms, e0, e1));
+      if (rep == 1 && ms < best) {
+        best = ms;
+        pick = nt;
       }
-  }
-  if (a.use_cells) launch_cells(a, ctx->d, ncell0, st);
+    }
   ctx->real_threads = pick;
-  ctx->cell_h = hpick;
   return ERMOD_OK;
 }
 
@@ -988,7 +970,7 @@ static int frame_enqueue(ermod_ctx* ctx, const FramePlan& fp, cudaStream_t st, b
   CK(cudaMemsetAsync(d.status, 0, sizeof(DevStatus), st));
   launch_prepare_solvent(a, d, st);
   launch_cells(a, d, fp.ncell, st);
-  nl += 1 + (a.slvmax > 0 ? (a.use_cells ? 3 : 2) : 0);
+  nl += 1 + (a.slvmax > 0 ? (a.use_cells ? 4 : 3) : 0);
   M(kStPrep);
   // ---- targets ----
   if (refs && fp.prop_gv > 0) {
@@ -1042,7 +1024,7 @@ static int frame_enqueue(ermod_ctx* ctx, const FramePlan& fp, cudaStream_t st, b
   for (int bb = 0; bb < ctx->maxdst; bb += ctx->batch) {
     const int nbatch = std::min(ctx->batch, ctx->maxdst - bb);
     if (ctx->real_threads == 0) {
-      const int rc = tune_real(ctx, a, fp.ncell, nbatch, st);
+      const int rc = tune_real(ctx, a, nbatch, st);
       if (rc != ERMOD_OK) return rc;
     }
     // Real space beside the PME chain: k_real on the second stream, joined before binning (the

@@ -42,7 +42,7 @@ struct FrameArgs {
   int ljtype_max;
   int pme;
   double pivol;                    // pi / screen^2 / volume (residual terms, engproc.F90:974,994)
-  // cell list (cuboid periodic boxes)
+  // cells of the molecules' spatial order (cuboid periodic boxes)
   int use_cells, nc[3];
   float ch[3];                     // cell edge lengths
   float rcut;                      // max(elecut, upljcut): beyond it every pair term is zero
@@ -126,13 +126,14 @@ struct DeviceState {
   float* spl = nullptr;      // [natoms*3*order]
   int4* grd = nullptr;       // [natoms]
   float* grec = nullptr;     // [natoms*kRecWords] order-4 gather records, on meshes gather_rec_ok allows
-  int4* mrec = nullptr;      // [slvmax] {molecule, first atom, atoms, charge bits} in cell order
+  int4* mrec = nullptr;      // [slvmax] {molecule, first atom, atoms, charge bits} in spatial order
+  float4* sanch = nullptr;   // [slvmax] anchors in spatial order
+  float4* gsph = nullptr;    // [(slvmax + 31) / 32] sphere around each group of 32 molecules of that order
   float4* anchor = nullptr;  // [slvmax] first-site position, w = molecule extent
   int* cellof = nullptr;     // [slvmax]
   int* cellcount = nullptr;  // [ncell_cap]
   int* cellstart = nullptr;  // [ncell_cap+1]
   int* molsorted = nullptr;  // [slvmax]
-  float* rmol = nullptr;     // [1] max molecule extent
   // per frame: targets (insertions or soln solutes)
   float* ins_conf = nullptr; // [3*s*maxdst] staging of caller conformations
   float* insw_in = nullptr;  // [maxdst]

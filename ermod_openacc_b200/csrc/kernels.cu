@@ -3,8 +3,8 @@
 // Stage map (reference routine each kernel replaces):
 //   k_prepare_solvent  normalize_periodic (realcal.F90:859-896) + solvent splines
 //                      (recpcal_prepare_solvent / calc_spline_molecule, recpcal.F90:340-357, 504-538)
-//   k_anchor / k_cell_*  cell list of solvent molecules (no reference counterpart:
-//                      the reference evaluates every site pair, realcal.F90:257-361)
+//   k_anchor / k_cell_* / k_mol_groups  spatial order of the solvent molecules (no reference
+//                      counterpart: the reference evaluates every site pair, realcal.F90:257-361)
 //   k_insert           instslt('proc') for uniform insertion (insertion.F90:38-375)
 //   k_selfreal         realcal_self(_refs) in FP64 (realcal.F90:669-771)
 //   k_real             realcal_refs / realcal_soln / realcal_bare (realcal.F90:51-666)
@@ -106,7 +106,9 @@ void launch_prepare_solvent(const FrameArgs& a, const DeviceState& d, cudaStream
 }
 
 // ---------------------------------------------------------------------------
-// cell list of solvent molecules, keyed by the normalised first site
+// the solvent molecules in spatial order: cells of about four molecules, keyed by the
+// normalised first site, numbered in blocks of 2 x 2 x 2 cells, so that 32 consecutive
+// molecules of the order are a compact group
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ int cell_coord(float x, float h, int n) {
   int c = (int)floorf(x / h);
@@ -114,8 +116,7 @@ __device__ __forceinline__ int cell_coord(float x, float h, int n) {
 }
 
 __global__ void k_anchor(FrameArgs a, const int* __restrict__ molbeg, const float4* __restrict__ slvn,
-                         float4* __restrict__ anchor, int* __restrict__ cellof, int* __restrict__ cellcount,
-                         float* rmol) {
+                         float4* __restrict__ anchor, int* __restrict__ cellof, int* __restrict__ cellcount) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= a.slvmax) return;
   const int b0 = molbeg[k], b1 = molbeg[k + 1];
@@ -128,12 +129,12 @@ __global__ void k_anchor(FrameArgs a, const int* __restrict__ molbeg, const floa
     ext = fmaxf(ext, sqrtf(dx * dx + dy * dy + dz * dz));
   }
   anchor[k] = make_float4(p0.x, p0.y, p0.z, ext);
-  atomicMax((int*)rmol, __float_as_int(ext));
   if (a.use_cells) {
     const int cx = cell_coord(p0.x, a.ch[0], a.nc[0]);
     const int cy = cell_coord(p0.y, a.ch[1], a.nc[1]);
     const int cz = cell_coord(p0.z, a.ch[2], a.nc[2]);
-    const int cid = (cz * a.nc[1] + cy) * a.nc[0] + cx;
+    const int bx = (a.nc[0] + 1) >> 1, by = (a.nc[1] + 1) >> 1;
+    const int cid = ((((cz >> 1) * by + (cy >> 1)) * bx + (cx >> 1)) << 3) | (cz & 1) << 2 | (cy & 1) << 1 | (cx & 1);
     cellof[k] = cid;
     atomicAdd(&cellcount[cid], 1);
   }
@@ -178,28 +179,57 @@ __global__ void k_iota(int n, int* __restrict__ out) {
   if (k < n) out[k] = k;
 }
 
-// the gather's molecule records in cell order: {molecule, first atom, atoms, charge bits}
-__global__ void k_mol_records(int slvmax, const int* __restrict__ molsorted, const int* __restrict__ molbeg,
-                              const float* __restrict__ molq, int4* __restrict__ mrec) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= slvmax) return;
-  const int k = molsorted[m];
-  mrec[m] = make_int4(k, molbeg[k], molbeg[k + 1] - molbeg[k], __float_as_int(molq[k]));
+// Per molecule in spatial order, its record {molecule, first atom, atoms, charge bits} (gather,
+// real space) and its anchor; per group of 32 consecutive molecules a sphere around all their
+// sites, for the real-space kernel's culling.  A warp per group.
+__global__ void k_mol_groups(FrameArgs a, const int* __restrict__ molsorted, const int* __restrict__ molbeg,
+                             const float* __restrict__ molq, const float4* __restrict__ anchor,
+                             int4* __restrict__ mrec, float4* __restrict__ sanch, float4* __restrict__ gsph) {
+  const int m = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+  const bool on = m < a.slvmax;
+  float4 an = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (on) {
+    const int k = molsorted[m];
+    mrec[m] = make_int4(k, molbeg[k], molbeg[k + 1] - molbeg[k], __float_as_int(molq[k]));
+    an = anchor[k];
+    sanch[m] = an;
+  }
+  // centre: the first anchor plus the mean displacement from it
+  const float ox = __shfl_sync(0xffffffffu, an.x, 0), oy = __shfl_sync(0xffffffffu, an.y, 0),
+              oz = __shfl_sync(0xffffffffu, an.z, 0);
+  float dx = an.x - ox, dy = an.y - oy, dz = an.z - oz;
+  min_image(a.g, dx, dy, dz);
+  if (!on) dx = dy = dz = 0.f;
+  const float n = (float)__popc(__ballot_sync(0xffffffffu, on));
+  float cx = dx, cy = dy, cz = dz;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    cx += __shfl_xor_sync(0xffffffffu, cx, o);
+    cy += __shfl_xor_sync(0xffffffffu, cy, o);
+    cz += __shfl_xor_sync(0xffffffffu, cz, o);
+  }
+  if (n == 0.f) return;
+  cx = ox + cx / n; cy = oy + cy / n; cz = oz + cz / n;
+  dx = an.x - cx; dy = an.y - cy; dz = an.z - cz;
+  min_image(a.g, dx, dy, dz);
+  float r = on ? sqrtf(dx * dx + dy * dy + dz * dz) + an.w : 0.f;
+  if (r != r) r = INFINITY;      // a coordinate that is no number is left to the pair loop
+  r = warp_max(r);
+  if (lane == 0) gsph[m >> 5] = make_float4(cx, cy, cz, r);
 }
 
 void launch_cells(const FrameArgs& a, const DeviceState& d, int ncell, cudaStream_t s) {
   if (a.slvmax <= 0) return;
-  cudaMemsetAsync(d.rmol, 0, sizeof(float), s);
   if (a.use_cells) cudaMemsetAsync(d.cellcount, 0, sizeof(int) * ncell, s);
-  k_anchor<<<(a.slvmax + 255) / 256, 256, 0, s>>>(a, d.molbeg, d.slvn, d.anchor, d.cellof, d.cellcount, d.rmol);
+  k_anchor<<<(a.slvmax + 255) / 256, 256, 0, s>>>(a, d.molbeg, d.slvn, d.anchor, d.cellof, d.cellcount);
   if (a.use_cells) {
     k_cell_scan<<<1, 1024, 0, s>>>(ncell, d.cellcount, d.cellstart);
     k_cell_fill<<<(a.slvmax + 255) / 256, 256, 0, s>>>(a.slvmax, d.cellof, d.cellcount, d.molsorted);
   } else {
     k_iota<<<(a.slvmax + 255) / 256, 256, 0, s>>>(a.slvmax, d.molsorted);
   }
-  if (a.pme && d.mrec)
-    k_mol_records<<<(a.slvmax + 255) / 256, 256, 0, s>>>(a.slvmax, d.molsorted, d.molbeg, d.molq, d.mrec);
+  k_mol_groups<<<(a.slvmax + 127) / 128, 128, 0, s>>>(a, d.molsorted, d.molbeg, d.molq, d.anchor, d.mrec, d.sanch,
+                                                      d.gsph);
 }
 
 // ---------------------------------------------------------------------------
@@ -735,214 +765,314 @@ void launch_selfreal(const FrameArgs& a, const DeviceState& d, int first, int co
 }
 
 // ---------------------------------------------------------------------------
-// real space: one CTA per target, warps over the cells around it
+// real space: CTAs per target, warps over the groups of 32 molecules around it
 // ---------------------------------------------------------------------------
-constexpr int kRealMaxThreads = 512;
+constexpr int kRealMaxThreads = 256;
+constexpr int kRealTile = 16;      // solute sites a lane tests at a time
+// Energies keep the bits that the library's results have had: the squared distance is rounded as
+// (y^2 + x^2) + z^2 for solutes of up to this many sites and as (x^2 + y^2) + z^2 above.
+constexpr int kRealYFirst = 64;
 
-// Small solutes: the lanes of a warp test 32 candidate molecules at a time
-// against the cutoff sphere and queue those in range (ballot, per-warp queue
-// in shared memory); each batch of up to 32 is then evaluated a molecule per
-// lane, all its (site, atom) pairs in turn.  WIDE (large solutes): a warp per
-// molecule, lanes over the solute sites, the molecule's atoms in turn, and a
-// warp-shuffle reduction.  Either way a molecule's energy is one fixed-order
-// FP64 sum.  The solute sites, the LJ tables and the queues sit in shared
-// memory (dynamic: s float4 + s int + 2 ljmax^2 float + 64 int per warp).
-template <bool WIDE>
-__global__ void __launch_bounds__(kRealMaxThreads) k_real(FrameArgs a, int base, int chunk,
+// A molecule is taken by LPM lanes, its sites dealt out to them in turn; each lane adds its pair
+// energies in FP64 in a fixed order and the LPM sums are added in a fixed tree, so a molecule's
+// energy does not depend on the block, the batch or the order it is met in.
+//
+// The solute is walked in tiles of 16 LPM consecutive sites.  Per tile, a warp tests 32 groups'
+// spheres at once against the tile's; the molecules of a group in reach are tested a lane each,
+// and those in reach are queued.  For each batch of 32 / LPM queued molecules a lane tests its 16
+// sites against three atoms (plain differences from the tile's centre, slightly wider than the
+// cutoff) and keeps the hits as bits; the warp's hits are then listed in shared memory and
+// evaluated 32 a turn, whoever's they are, at the single call of pair_energy, which applies the
+// exact cutoff; each lane last adds up its own energies.
+//
+// Why: the pair energy (about 200 instructions, erfcf and the exact roots and quotients most of
+// them) bounds the kernel, at 65 % of the issue slots.  A warp that evaluated its lanes' pairs in
+// lockstep spent a pair energy wherever one lane needed it: 15 of 32 lanes were active, and of a
+// chain's sites 94 % lay beyond the cutoff of the molecules in reach.  Listing the hits keeps 31
+// lanes active; the spheres per tile leave out most of what a long chain does not reach.
+// Measured before and with it, real-space stage of one frame: 12-site ring, 2000 insertions into
+// 4096 waters 0.43 -> 0.29 ms; 60-site chain, 2048 into 32,768 waters 7.1 -> 2.1 ms; 200 sites,
+// 4000 into 4096 waters 24.2 -> 8.8 ms; one 60-site solute in solution, 4096 waters (one CTA
+// before, 16 lanes a molecule over the whole chip now) 0.57 -> 0.026 ms.
+struct RealWarp {
+  float4 atom[3 * 32];
+  int lj[3 * 32];
+  int slot[32 * 3 * kRealTile * 17 / 16];
+  int queue[64];
+};
+// place of hit p: lanes whose runs of up to 16 hits start 16 apart would share two banks
+__device__ __forceinline__ int skew(int p) { return p + (p >> 4); }
+
+template <int LPM>
+__global__ void __launch_bounds__(kRealMaxThreads, 3) k_real(FrameArgs a, int base, int ny,
     const float4* __restrict__ tgt_n, const float4* __restrict__ tgt_c, const int* __restrict__ tgt_mol,
     const int* __restrict__ slt_lj_tab, const int* __restrict__ molbeg, const float4* __restrict__ slvn,
     const int* __restrict__ atom_lj, const float* __restrict__ ljene, const float* __restrict__ ljlensq,
-    const float4* __restrict__ anchor, const int* __restrict__ cellstart, const int* __restrict__ molsorted,
-    const float* __restrict__ rmol_p, double* __restrict__ E) {
+    const int4* __restrict__ mrec, const float4* __restrict__ sanch, const float4* __restrict__ gsph,
+    double* __restrict__ E) {
   extern __shared__ __align__(16) unsigned char rsm_real[];
+  constexpr int NB = 32 / LPM;                 // molecules of a batch
+  constexpr int TS = kRealTile * LPM;          // sites of a tile
   const int b = blockIdx.x, cnt = base + b, s = a.nsite;
-  const int ljmax = a.ljtype_max;
-  float4* ss = (float4*)rsm_real;
-  int* slj = (int*)(ss + s);
-  float* lje = (float*)(slj + s);
+  const int ljmax = a.ljtype_max, nt = (s + TS - 1) / TS;
+  float4* ss = (float4*)rsm_real;              // [s] site positions, charges
+  float4* rel = ss + s;                        // [nt TS] positions from the tile's centre, w = LJ type
+  float4* tile = rel + nt * TS;                // [nt] centre, radius
+  float* lje = (float*)(tile + nt);
   float* ljs = lje + ljmax * ljmax;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  // this warp's batch atoms and LJ types, its hits (later their energies), its queue of molecules in reach
+  RealWarp& W = ((RealWarp*)(((uintptr_t)(ljs + ljmax * ljmax) + 15) & ~(uintptr_t)15))[warp];
+  float4* satom = W.atom;
+  int *slj = W.lj, *slot = W.slot, *q = W.queue;
+  const unsigned below = (1u << lane) - 1u;
   const float4* tn = tgt_n + (size_t)cnt * s;
-  for (int i = threadIdx.x; i < s; i += blockDim.x) {
-    ss[i] = tn[i];
-    slj[i] = slt_lj_tab ? slt_lj_tab[i] : 0;
-  }
+  for (int i = threadIdx.x; i < s; i += blockDim.x) ss[i] = tn[i];
   for (int i = threadIdx.x; i < ljmax * ljmax; i += blockDim.x) {
     lje[i] = ljene[i];
     ljs[i] = ljlensq[i];
   }
   const int excl = tgt_mol ? tgt_mol[cnt] : -1;
   // soln: solute site LJ types come from the solute molecule's atoms
-  if (excl >= 0)
-    for (int i = threadIdx.x; i < s; i += blockDim.x) slj[i] = atom_lj[molbeg[excl] + i];
+  const int* site_lj = excl >= 0 ? atom_lj + molbeg[excl] : slt_lj_tab;
   __syncthreads();
-  const float4 c = tgt_c[cnt];
-  const float rmol = *rmol_p;
+  const bool metric = !a.g.periodic || a.g.cuboid;     // distances obey the triangle inequality
   const float margin = 1.0e-2f;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  // a warp per tile: centre (the mean site), the sites' offsets from it, radius
+  for (int t = warp; t < nt; t += nw) {
+    const int t0 = t * TS, len = min(TS, s - t0);
+    const float4 o = ss[t0];
+    float cx = 0.f, cy = 0.f, cz = 0.f;
+    for (int i = lane; i < len; i += 32) {
+      float x = ss[t0 + i].x - o.x, y = ss[t0 + i].y - o.y, z = ss[t0 + i].z - o.z;
+      min_image(a.g, x, y, z);
+      cx += x; cy += y; cz += z;
+    }
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) {
+      cx += __shfl_xor_sync(0xffffffffu, cx, w);
+      cy += __shfl_xor_sync(0xffffffffu, cy, w);
+      cz += __shfl_xor_sync(0xffffffffu, cz, w);
+    }
+    const float inv = 1.0f / (float)len;
+    cx = o.x + cx * inv; cy = o.y + cy * inv; cz = o.z + cz * inv;
+    float r = 0.f;
+    bool bad = false;                                  // a coordinate that is no number: keep every pair
+    for (int i = lane; i < TS; i += 32) {
+      float x = 0.f, y = 0.f, z = 0.f;
+      int lj = 0;
+      if (i < len) {
+        x = ss[t0 + i].x - cx; y = ss[t0 + i].y - cy; z = ss[t0 + i].z - cz;
+        min_image(a.g, x, y, z);
+        const float d = sqrtf(x * x + y * y + z * z);
+        r = fmaxf(r, d);
+        bad |= d != d;
+        lj = site_lj ? site_lj[t0 + i] : 0;
+      }
+      rel[t0 + i] = make_float4(x, y, z, __int_as_float(lj));
+    }
+    r = warp_max(bad ? INFINITY : r);
+    if (lane == 0) tile[t] = make_float4(cx, cy, cz, r);
+  }
+  __syncthreads();
   // pairs beyond rcut (>= elecut and > upljcut) are zero; the slack keeps r == rcut with pair_energy
   const float rskip2 = a.rcut * a.rcut * 1.0001f;
+  const float rtest = a.rcut * 1.0001f + 2.0e-3f, rtest2 = rtest * rtest;
+  const float halfbox = fminf(a.g.half[0], fminf(a.g.half[1], a.g.half[2]));
+  const int sub = lane % LPM;
+  const bool yfirst = s <= kRealYFirst;
 
-  // candidate k (-1: none) can have a site pair within the cutoff
-  auto in_range = [&](int k) {
-    if (k < 0 || k == excl) return false;
-    const float4 an = anchor[k];
-    float dx = an.x - c.x, dy = an.y - c.y, dz = an.z - c.z;
-    min_image(a.g, dx, dy, dz);
-    const float lim = a.rcut + c.w + an.w + margin;
-    return !(dx * dx + dy * dy + dz * dz > lim * lim);
-  };
-  // WIDE: molecule k by the whole warp, lanes over the solute sites
-  auto do_mol = [&](int k) {
-    if (!in_range(k)) return;  // every site pair beyond the cutoff
-    const int b0 = molbeg[k], nj = molbeg[k + 1] - b0;
-    double acc = 0.0;
-    for (int js = 0; js < nj; ++js) {
-      const float4 xj = slvn[b0 + js];
-      const int lj = atom_lj[b0 + js];
-      for (int is = lane; is < s; is += 32) {
-        const float4 xi = ss[is];
-        float ex = xi.x - xj.x, ey = xi.y - xj.y, ez = xi.z - xj.z;
-        min_image(a.g, ex, ey, ez);
-        const float dis2 = ex * ex + ey * ey + ez * ez;
-        if (dis2 > rskip2) continue;
-        const int li = slj[is];
-        acc += (double)pair_energy(a.pp, dis2, lje[lj * ljmax + li], ljs[lj * ljmax + li], xi.w * xj.w);
+  // work items: a group of 32 molecules in LPM parts of NB; a warp keeps its items for every tile
+  const int items = ((a.slvmax + 31) >> 5) * LPM, stride = ny * nw;
+  const float4 c = tgt_c[cnt];
+  for (int t = 0; t < nt; ++t) {
+    const float4 tc = metric ? tile[t] : c;             // the sphere that groups and molecules are tested against
+    const int t0 = t * TS + sub;
+    const int nv = min(kRealTile, (s - t0 + LPM - 1) / LPM);        // sites of this lane (may be < 1)
+    const int nvu = min(kRealTile, (s - t * TS + LPM - 1) / LPM);   // of the lane with most
+    // differences from the tile's centre are the nearest images' wherever a pair is inside the
+    // cutoff, as long as the cutoff sphere around the tile is narrower than the box
+    const bool plain = !a.g.periodic || (a.g.cuboid && a.rcut + tc.w + margin < halfbox);
+    int ibase = blockIdx.y * nw + warp;
+    unsigned imask = 0u;          // items ibase - 32 stride + j stride (j a set bit) still to take
+    int qn = 0;
+    for (;;) {
+      while (qn < NB) {
+        while (imask == 0u && ibase < items) {
+          const int it = ibase + lane * stride;
+          bool in = it < items;
+          if (in && metric) {
+            const float4 gs = gsph[it / LPM];
+            float dx = gs.x - tc.x, dy = gs.y - tc.y, dz = gs.z - tc.z;
+            min_image(a.g, dx, dy, dz);
+            const float lim = a.rcut + tc.w + gs.w + margin;
+            in = !(dx * dx + dy * dy + dz * dz > lim * lim);
+          }
+          imask = __ballot_sync(0xffffffffu, in);
+          ibase += 32 * stride;
+        }
+        if (imask == 0u) break;
+        const int j = __ffs(imask) - 1;
+        imask &= imask - 1u;
+        const int it = ibase - 32 * stride + j * stride;
+        const int m = (it / LPM) * 32 + lane;
+        // a molecule can have a site pair within the cutoff
+        bool in = m < a.slvmax && (LPM == 1 || lane / NB == it % LPM);
+        if (in) {
+          const float4 an = sanch[m];
+          float dx = an.x - tc.x, dy = an.y - tc.y, dz = an.z - tc.z;
+          min_image(a.g, dx, dy, dz);
+          const float lim = a.rcut + tc.w + an.w + margin;
+          in = !(dx * dx + dy * dy + dz * dz > lim * lim) && mrec[m].x != excl;
+        }
+        const unsigned bal = __ballot_sync(0xffffffffu, in);
+        if (in) q[qn + __popc(bal & below)] = m;
+        qn += __popc(bal);
       }
-    }
-    acc = warp_sum(acc);
-    if (lane == 0) E[(size_t)b * a.slvmax + k] = acc;
-  };
-
-  // the cells around the target (all cells when the range covers the box)
-  (void)rmol;
-  int lo[3] = {0, 0, 0}, n[3] = {1, 1, 1};
-  int total;
-  if (a.use_cells) {
-    const float R = a.rcut + c.w + rmol + margin;
-    const float cc[3] = {c.x, c.y, c.z};
-    for (int d3 = 0; d3 < 3; ++d3) {
-      lo[d3] = (int)floorf((cc[d3] - R) / a.ch[d3]);
-      const int hi = (int)floorf((cc[d3] + R) / a.ch[d3]);
-      n[d3] = hi - lo[d3] + 1;
-      if (n[d3] >= a.nc[d3]) { lo[d3] = 0; n[d3] = a.nc[d3]; }
-    }
-    total = n[0] * n[1] * n[2];
-  } else {
-    total = (a.slvmax + 7) / 8;   // without cells: runs of 8 molecules
-  }
-  auto cell_id = [&](int t) {
-    const int ix = t % n[0], iy = (t / n[0]) % n[1], iz = t / (n[0] * n[1]);
-    int cx = (lo[0] + ix) % a.nc[0]; if (cx < 0) cx += a.nc[0];
-    int cy = (lo[1] + iy) % a.nc[1]; if (cy < 0) cy += a.nc[1];
-    int cz = (lo[2] + iz) % a.nc[2]; if (cz < 0) cz += a.nc[2];
-    return (cz * a.nc[1] + cy) * a.nc[0] + cx;
-  };
-
-  if (WIDE) {
-    for (int t = warp; t < total; t += nw) {
-      if (a.use_cells) {
-        const int cid = cell_id(t);
-        for (int m = cellstart[cid]; m < cellstart[cid + 1]; ++m) do_mol(molsorted[m]);
-      } else {
-        for (int k = 8 * t; k < min(8 * t + 8, a.slvmax); ++k) do_mol(k);
+      if (qn == 0) break;
+      __syncwarp();
+      // the last NB molecules of the queue; lanes past its end take its first entry and store nothing
+      const int nbm = min(NB, qn), mine = lane / LPM;
+      const bool live = mine < nbm;
+      const int4 mr = mrec[q[qn - nbm + (live ? mine : 0)]];
+      qn -= nbm;
+      const int njmax = __reduce_max_sync(0xffffffffu, mr.z);
+      double* const out = E + (size_t)b * a.slvmax + mr.x;
+      const double before = t > 0 && live && sub == 0 ? *out : 0.0;
+      double acc = 0.0;
+      for (int js0 = 0; js0 < njmax; js0 += 3) {
+        float4 xj[3];
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < 3; ++u) {
+          const int at = mr.y + max(0, min(js0 + u, mr.z - 1));
+          xj[u] = slvn[at];
+          satom[u * 32 + lane] = xj[u];
+          slj[u * 32 + lane] = atom_lj[at];
+        }
+        unsigned hit[3] = {0u, 0u, 0u};
+        if (plain) {
+          float px[3], py[3], pz[3];
+#pragma unroll
+          for (int u = 0; u < 3; ++u) {
+            px[u] = xj[u].x - tc.x; py[u] = xj[u].y - tc.y; pz[u] = xj[u].z - tc.z;
+            min_image(a.g, px[u], py[u], pz[u]);
+          }
+#pragma unroll 4
+          for (int i = 0; i < nvu; ++i) {
+            const float4 r = rel[t0 + i * LPM];
+#pragma unroll
+            for (int u = 0; u < 3; ++u) {
+              const float dx = px[u] - r.x, dy = py[u] - r.y, dz = pz[u] - r.z;
+              if (!(dx * dx + dy * dy + dz * dz > rtest2)) hit[u] |= 1u << i;
+            }
+          }
+        } else {
+          for (int i = 0; i < nv; ++i) {
+            const float4 r = ss[t0 + i * LPM];
+#pragma unroll
+            for (int u = 0; u < 3; ++u) {
+              float dx = r.x - xj[u].x, dy = r.y - xj[u].y, dz = r.z - xj[u].z;
+              min_image(a.g, dx, dy, dz);
+              if (!(dx * dx + dy * dy + dz * dz > rskip2)) hit[u] |= 1u << i;
+            }
+          }
+        }
+        const unsigned valid = live && nv > 0 && js0 < mr.z ? (1u << nv) - 1u : 0u;   // nv <= 16
+        hit[0] &= valid;
+        hit[1] &= js0 + 1 < mr.z ? valid : 0u;
+        hit[2] &= js0 + 2 < mr.z ? valid : 0u;
+        // the warp's hits, in (atom, lane, site) order, into `slot`
+        int n = 0, at0[3];
+#pragma unroll
+        for (int u = 0; u < 3; ++u) {
+          const int cnt_u = __popc(hit[u]);
+          int sum = cnt_u;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += v;
+          }
+          at0[u] = n + sum - cnt_u;
+          n += __shfl_sync(0xffffffffu, sum, 31);
+        }
+        if (n == 0) continue;
+#pragma unroll
+        for (int u = 0; u < 3; ++u) {
+          int p = at0[u];
+          for (unsigned w = hit[u]; w; w &= w - 1u, ++p) slot[skew(p)] = lane | u << 5 | (__ffs(w) - 1) << 7;
+        }
+        __syncwarp();
+        // 32 pairs a turn, whoever's they are; each energy takes its hit's place
+        for (int p = lane; p < n; p += 32) {
+          const int e = slot[skew(p)], o = e & 31, u = (e >> 5) & 3, is = t * TS + (e >> 7) * LPM + o % LPM;
+          const float4 xi = ss[is], x = satom[u * 32 + o];
+          const int l = slj[u * 32 + o], li = __float_as_int(rel[is].w);
+          float ex = xi.x - x.x, ey = xi.y - x.y, ez = xi.z - x.z;
+          min_image(a.g, ex, ey, ez);
+          // the order of the squares is part of a result's bits: y first up to kRealYFirst sites
+          const float e0 = yfirst ? ey : ex, e1 = yfirst ? ex : ey;
+          const float dis2 = __fmaf_rn(ez, ez, __fmaf_rn(e1, e1, __fmul_rn(e0, e0)));
+          float v = 0.0f;
+          if (!(dis2 > rskip2)) v = pair_energy(a.pp, dis2, lje[l * ljmax + li], ljs[l * ljmax + li], xi.w * x.w);
+          slot[skew(p)] = __float_as_int(v);
+        }
+        __syncwarp();
+        // each lane adds its own
+#pragma unroll
+        for (int u = 0; u < 3; ++u)
+          for (int p = at0[u], e = p + __popc(hit[u]); p < e; ++p) acc += (double)__int_as_float(slot[skew(p)]);
       }
+#pragma unroll
+      for (int o = LPM / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+      if (live && sub == 0) *out = before + acc;
+      __syncwarp();                 // the next tile's lanes read these sums
     }
-    return;
-  }
-
-  // Small solutes.  Each lane walks its own cells (t = warp * 32 + lane, then every
-  // nw * 32-th), so a ballot step tests up to 32 candidates; molecules in range go to
-  // the warp's queue, and every batch of up to 32 is evaluated a molecule per lane at the
-  // single call site below (one compiled body: a molecule's sum does not depend on which
-  // batch it lands in, and the order of molecules within a cell is not fixed).
-  int* q = (int*)(ljs + ljmax * ljmax) + warp * 64;   // this warp's queue of molecules in range
-  int qn = 0;                                          // queued (warp-uniform)
-  int tc = warp * 32 + lane, m = 0, m1 = 0;            // this lane's cell cursor and candidate range
-  auto next_cell = [&]() {
-    while (m >= m1 && tc < total) {
-      if (a.use_cells) {
-        const int cid = cell_id(tc);
-        m = cellstart[cid];
-        m1 = cellstart[cid + 1];
-      } else {
-        m = 8 * tc;
-        m1 = min(m + 8, a.slvmax);
-      }
-      tc += nw * 32;
-    }
-  };
-  next_cell();
-  for (;;) {
-    bool more = __any_sync(0xffffffffu, m < m1);
-    while (qn < 32 && more) {
-      int kl = -1;
-      if (m < m1) {
-        kl = a.use_cells ? molsorted[m] : m;
-        if (++m >= m1) next_cell();
-      }
-      const bool in = in_range(kl);
-      const unsigned bal = __ballot_sync(0xffffffffu, in);
-      if (in) q[qn + __popc(bal & ((1u << lane) - 1u))] = kl;
-      qn += __popc(bal);
-      more = __any_sync(0xffffffffu, m < m1);
-    }
-    __syncwarp();
-    if (qn == 0) break;
-    // lanes past the queue's end repeat entry 0 and store nothing
-    const int k = q[lane < qn ? lane : 0];
-    const int b0 = molbeg[k], nj = molbeg[k + 1] - b0;
-    double acc = 0.0;
-    for (int is = 0; is < s; ++is) {
-      const float4 xi = ss[is];
-      const int li = slj[is];
-      for (int js = 0; js < nj; ++js) {
-        const float4 xj = slvn[b0 + js];
-        float ex = xi.x - xj.x, ey = xi.y - xj.y, ez = xi.z - xj.z;
-        min_image(a.g, ex, ey, ez);
-        const float dis2 = ex * ex + ey * ey + ez * ez;
-        if (dis2 > rskip2) continue;
-        const int lj = atom_lj[b0 + js];
-        acc += (double)pair_energy(a.pp, dis2, lje[lj * ljmax + li], ljs[lj * ljmax + li], xi.w * xj.w);
-      }
-    }
-    if (lane < qn) E[(size_t)b * a.slvmax + k] = acc;
-    __syncwarp();
-    if (lane < qn - 32) q[lane] = q[32 + lane];
-    qn = qn > 32 ? qn - 32 : 0;
-    __syncwarp();
   }
 }
 
-// Solutes above this many sites run the WIDE real-space variant (a warp per molecule, lanes
-// over the sites); up to it, a molecule a lane is faster (measured on ring-recipe solutes of
-// 24 to 60 sites in 4096 waters: real space 3.0 -> 2.0 ms at 28 sites, 4.3 -> 2.9 at 40).
-constexpr int kRealWideSites = 64;
+// Lanes a molecule: one, unless the targets' molecules give fewer than 16 warps an SM (a solution
+// frame has one target); then four or sixteen share a molecule's sites.  One 60-site solute in
+// 4096 waters: 0.08 ms with one lane a molecule, 0.026 with sixteen.  A rule on the context's
+// sizes alone, so every batch of a context, and a context inside a batch, sums alike.
+int real_lpm(const FrameArgs& a) {
+  int lpm = 1;
+  while (lpm < 16 && 2 * lpm <= a.nsite && (double)a.maxdst * a.slvmax * lpm < 148.0 * 16 * 32) lpm *= 4;
+  return lpm;
+}
 
-size_t real_smem(const FrameArgs& a) {
-  return (sizeof(float4) + sizeof(int)) * (size_t)a.nsite + 2 * sizeof(float) * (size_t)a.ljtype_max * a.ljtype_max +
-         sizeof(int) * 64 * (kRealMaxThreads / 32);
+size_t real_smem(const FrameArgs& a, int lpm, int threads) {
+  const size_t ts = (size_t)kRealTile * lpm, nt = (a.nsite + ts - 1) / ts;
+  return sizeof(float4) * (a.nsite + nt * ts + nt) + 2 * sizeof(float) * (size_t)a.ljtype_max * a.ljtype_max + 16 +
+         sizeof(RealWarp) * (threads / 32);
 }
 
 int setup_real_smem(const FrameArgs& a) {
-  const int b = (int)real_smem(a);
-  if (raise_smem_limit(k_real<true>, (size_t)b) != cudaSuccess) return -1;
-  if (raise_smem_limit(k_real<false>, (size_t)b) != cudaSuccess) return -1;
-  return 0;
+  const int lpm = real_lpm(a);
+  cudaError_t e = lpm == 1   ? raise_smem_limit(k_real<1>, real_smem(a, 1, kRealMaxThreads))
+                  : lpm == 4 ? raise_smem_limit(k_real<4>, real_smem(a, 4, kRealMaxThreads))
+                             : raise_smem_limit(k_real<16>, real_smem(a, 16, kRealMaxThreads));
+  return e == cudaSuccess ? 0 : -1;
 }
 
-// `threads` (a multiple of 32, <= kRealMaxThreads) only changes how many warps
-// share a target's molecules: each molecule's energy is one warp's fixed-order
-// sum whatever the block size.
+// `threads` (a multiple of 32, <= kRealMaxThreads) only changes how the warps share a target's
+// molecules.  Several CTAs a target where there are few, up to eight an SM in all: 32 an SM end
+// more evenly (2000 insertions of the ring 0.27 against 0.29 ms) but leave a warp too few of a
+// tile's molecules to fill its batches (32,768 waters 2.6 against 2.1 ms, 200 sites 9.3 against 8.8).
 void launch_real(const FrameArgs& a, const DeviceState& d, int base, int nb, int chunk, int threads, cudaStream_t s) {
   cudaMemsetAsync(d.E, 0, sizeof(double) * (size_t)a.slvmax * chunk, s);
   if (nb <= 0) return;  // `chunk` is the row stride of E: the batch size
   if (threads <= 0 || threads > kRealMaxThreads || threads % 32) threads = 256;
-  const size_t sm = real_smem(a);
+  const int lpm = real_lpm(a), items = (a.slvmax + 31) / 32 * lpm;
+  const int ny = std::max(1, std::min((148 * 8 + nb - 1) / nb, (items + threads / 32 - 1) / (threads / 32)));
+  const size_t sm = real_smem(a, lpm, threads);
   // launch_k: a graph node of this launch keeps the stream's (lower) priority beside the PME chain
-#define ERM_REAL(W) launch_k(false, nb, threads, sm, s, k_real<W>, a, base, chunk, d.tgt_n, d.tgt_c, d.tgt_mol, \
-      d.slt_lj, d.molbeg, d.slvn, d.atom_lj, d.ljene, d.ljlensq, d.anchor, d.cellstart, d.molsorted, d.rmol, d.E)
-  if (a.nsite > kRealWideSites) ERM_REAL(true);
-  else ERM_REAL(false);
+#define ERM_REAL(L) launch_k(false, dim3(nb, ny), threads, sm, s, k_real<L>, a, base, ny, d.tgt_n, d.tgt_c, d.tgt_mol, \
+      d.slt_lj, d.molbeg, d.slvn, d.atom_lj, d.ljene, d.ljlensq, (const int4*)d.mrec, (const float4*)d.sanch, \
+      (const float4*)d.gsph, d.E)
+  if (lpm == 1) ERM_REAL(1);
+  else if (lpm == 4) ERM_REAL(4);
+  else ERM_REAL(16);
 #undef ERM_REAL
 }
 
