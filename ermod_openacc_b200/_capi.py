@@ -190,6 +190,10 @@ SIGNATURES = {
     "ermod_slvfe_delta_mu_ex": (C.c_int32, [C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int32, _f64p, _f64p,
                                             _f64p, _f64p, _i32p, C.c_double, _f64p, C.c_double,
                                             C.POINTER(ErmodSlvfeOpts), _f64p, _f64p, _i32p]),
+    "ermod_slvfe_delta_mu_layout": (C.c_int32, [C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int32, _f64p, _f64p,
+                                                _f64p, C.c_int32, _f64p, _i32p, C.c_double, _f64p, C.c_double,
+                                                C.POINTER(ErmodSlvfeOpts), _f64p, _f64p, _i32p]),
+    "ermod_slvfe_release": (None, []),
     "ermod_slvfe_last_error": (C.c_char_p, []),
 }
 

@@ -390,7 +390,9 @@ def delta_mu_gpu(edist, edens, ecorr, uvcrd, uvspec, temp_K: float, aveuv, slfen
     lib = A.load_library()
     rd = A.as_f64(edist)
     rr = A.as_f64(edens)
-    chi = np.asfortranarray(np.asarray(ecorr, dtype=np.float64))
+    chi = np.asarray(ecorr, dtype=np.float64)
+    if not chi.flags.f_contiguous:      # a C array goes to the device as it is and is transposed there
+        chi = np.ascontiguousarray(chi)
     crd = A.as_f64(uvcrd)
     spec = np.ascontiguousarray(uvspec, dtype=np.int32)
     av = A.as_f64(np.atleast_1d(aveuv))
@@ -399,10 +401,12 @@ def delta_mu_gpu(edist, edens, ecorr, uvcrd, uvspec, temp_K: float, aveuv, slfen
     tot = C.c_double()
     used = C.c_int32()
     opts = A.ErmodSlvfeOpts(functional=A.SLVFE_FUNCTIONALS[functional], evd=1 if evd else 0, et=float(et))
-    rc = lib.ermod_slvfe_delta_mu_ex(device, len(rd), nsp, group, inft, A.ptr(rd, C.c_double), A.ptr(rr, C.c_double),
-                                     chi.ctypes.data_as(C.POINTER(C.c_double)), A.ptr(crd, C.c_double),
-                                     A.ptr(spec, C.c_int32), kT_of(temp_K), A.ptr(av, C.c_double), float(slfeng),
-                                     C.byref(opts), A.ptr(out, C.c_double), C.byref(tot), C.byref(used))
+    rc = lib.ermod_slvfe_delta_mu_layout(device, len(rd), nsp, group, inft, A.ptr(rd, C.c_double),
+                                         A.ptr(rr, C.c_double), chi.ctypes.data_as(C.POINTER(C.c_double)),
+                                         0 if chi.flags.f_contiguous else 1, A.ptr(crd, C.c_double),
+                                         A.ptr(spec, C.c_int32), kT_of(temp_K), A.ptr(av, C.c_double),
+                                         float(slfeng), C.byref(opts), A.ptr(out, C.c_double), C.byref(tot),
+                                         C.byref(used))
     if info is not None:
         info["used_evd"] = bool(used.value)
     if rc != 0:

@@ -78,6 +78,18 @@ int32_t ermod_slvfe_delta_mu_ex(int32_t device, int32_t n, int32_t nsp, int32_t 
                                 double slfeng, const ermod_slvfe_opts* opts, double* chmpt, double* total,
                                 int32_t* used_evd);
 
+/* The same for chi_ref in either layout: element (i, j) at j * n + i (chi_row_major 0, as the
+ * entry points above take it) or at i * n + j (1, a C array). */
+int32_t ermod_slvfe_delta_mu_layout(int32_t device, int32_t n, int32_t nsp, int32_t group, int32_t inft,
+                                    const double* rho_sln, const double* rho_ref, const double* chi_ref,
+                                    int32_t chi_row_major, const double* crd, const int32_t* spec, double kT,
+                                    const double* aveuv, double slfeng, const ermod_slvfe_opts* opts,
+                                    double* chmpt, double* total, int32_t* used_evd);
+
+/* Calls keep up to two working buffers of at most 256 MB per device for the next call; this frees
+ * them.  No call may be running. */
+void ermod_slvfe_release(void);
+
 /* Name of the last error of ermod_slvfe_delta_mu on this thread. */
 const char* ermod_slvfe_last_error(void);
 
