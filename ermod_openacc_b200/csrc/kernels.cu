@@ -707,47 +707,78 @@ void launch_insert(const FrameArgs& a, const DeviceState& d, const int* stnum_de
                                                     d.tgt_c);
 }
 
+// a warp per solute: raw sites, normalised copies and the search sphere (finish_target's)
 __global__ void k_targets_soln(FrameArgs a, const int* __restrict__ tgt_mol, const int* __restrict__ molbeg,
                                const float* __restrict__ posraw, const float* __restrict__ atom_q,
                                float4* __restrict__ tgt_raw, float4* __restrict__ tgt_n, float4* __restrict__ tgt_c) {
-  const int cnt = blockIdx.x * blockDim.x + threadIdx.x;
+  const int cnt = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (cnt >= a.maxdst) return;
   const int k = tgt_mol[cnt], b0 = molbeg[k], s = a.nsite;
-  float4* out = tgt_raw + (size_t)cnt * s;
-  for (int i = 0; i < s; ++i)
-    out[i] = make_float4(posraw[3 * (b0 + i)], posraw[3 * (b0 + i) + 1], posraw[3 * (b0 + i) + 2], atom_q[b0 + i]);
-  finish_target(a, cnt, out, tgt_n + (size_t)cnt * s, tgt_c, nullptr);
+  float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
+  float rad = 0.0f;
+  for (int i0 = 0; i0 < s; i0 += 32) {
+    const int i = i0 + lane, at = b0 + min(i, s - 1);
+    const float4 r = make_float4(posraw[3 * at], posraw[3 * at + 1], posraw[3 * at + 2], atom_q[at]);
+    float x = r.x, y = r.y, z = r.z;
+    wrap_point(a.g, x, y, z);
+    if (i < s) {
+      tgt_raw[(size_t)cnt * s + i] = r;
+      tgt_n[(size_t)cnt * s + i] = make_float4(x, y, z, r.w);
+    }
+    if (i0 == 0) {
+      c.x = __shfl_sync(0xffffffffu, x, 0);
+      c.y = __shfl_sync(0xffffffffu, y, 0);
+      c.z = __shfl_sync(0xffffffffu, z, 0);
+    }
+    if (i > 0 && i < s) {
+      float dx = x - c.x, dy = y - c.y, dz = z - c.z;
+      min_image(a.g, dx, dy, dz);
+      rad = fmaxf(rad, sqrtf(dx * dx + dy * dy + dz * dz));
+    }
+  }
+  rad = warp_max(rad);
+  if (lane == 0) tgt_c[cnt] = make_float4(c.x, c.y, c.z, rad);
 }
 
 void launch_targets_soln(const FrameArgs& a, const DeviceState& d, const int*, cudaStream_t s) {
-  k_targets_soln<<<(a.maxdst + 127) / 128, 128, 0, s>>>(a, d.tgt_mol, d.molbeg, d.posraw, d.atom_q, d.tgt_raw,
-                                                          d.tgt_n, d.tgt_c);
+  k_targets_soln<<<(a.maxdst + 3) / 4, 128, 0, s>>>(a, d.tgt_mol, d.molbeg, d.posraw, d.atom_q, d.tgt_raw, d.tgt_n,
+                                                    d.tgt_c);
 }
 
-// realcal_self(_refs) (realcal.F90:669-771), FP64 on normalised coordinates
-__global__ void k_selfreal(FrameArgs a, int first, double screen, const float4* __restrict__ tgt_n,
-                           double* __restrict__ selfreal) {
+// realcal_self(_refs) (realcal.F90:669-771), FP64 on normalised coordinates: a CTA per target, the
+// site pairs (i < j) dealt to its threads in row order.  An FP64 erf is some 0.4 us of a thread, so
+// the pairs and not the rows are what is shared out.  With k_targets_soln, which a thread a solute
+// ran before: 60 sites in solution 56 -> 18 us.
+constexpr int kSelfThreads = 512;
+
+__global__ void __launch_bounds__(kSelfThreads) k_selfreal(FrameArgs a, int first, double screen,
+    const float4* __restrict__ tgt_n, double* __restrict__ selfreal) {
   const int cnt = first + blockIdx.x;
   const int s = a.nsite;
   const float4* x = tgt_n + (size_t)cnt * s;
   double acc = 0.0;
   const double sqpi = sqrt(kPi);
   for (int i = threadIdx.x; i < s; i += blockDim.x) acc -= (double)x[i].w * (double)x[i].w * screen / sqpi;
-  for (int i = 0; i < s; ++i)
-    for (int j = i + 1 + threadIdx.x; j < s; j += blockDim.x) {
-      float dx = x[i].x - x[j].x, dy = x[i].y - x[j].y, dz = x[i].z - x[j].z;
-      if (a.g.cuboid) {
-        dx = a.g.half[0] - fabsf(a.g.half[0] - fabsf(dx));
-        dy = a.g.half[1] - fabsf(a.g.half[1] - fabsf(dy));
-        dz = a.g.half[2] - fabsf(a.g.half[2] - fabsf(dz));
-      } else {
-        CellGeom g = a.g;
-        g.periodic = 1;
-        min_image(g, dx, dy, dz);
-      }
-      const double r = sqrt((double)dx * dx + (double)dy * dy + (double)dz * dz);
-      acc -= (double)x[i].w * (double)x[j].w * erf(screen * r) / r;
+  const int npair = s * (s - 1) / 2;
+  for (int e = threadIdx.x; e < npair; e += blockDim.x) {
+    // pair e: row i holds the s - 1 - i pairs from i (2 s - i - 1) / 2 on
+    int i = (int)(((double)(2 * s - 1) - sqrt((double)(2 * s - 1) * (2 * s - 1) - 8.0 * e)) * 0.5);
+    while (i > 0 && i * (2 * s - i - 1) / 2 > e) --i;
+    while ((i + 1) * (2 * s - i - 2) / 2 <= e) ++i;
+    const int j = i + 1 + e - i * (2 * s - i - 1) / 2;
+    float dx = x[i].x - x[j].x, dy = x[i].y - x[j].y, dz = x[i].z - x[j].z;
+    if (a.g.cuboid) {
+      dx = a.g.half[0] - fabsf(a.g.half[0] - fabsf(dx));
+      dy = a.g.half[1] - fabsf(a.g.half[1] - fabsf(dy));
+      dz = a.g.half[2] - fabsf(a.g.half[2] - fabsf(dz));
+    } else {
+      CellGeom g = a.g;
+      g.periodic = 1;
+      min_image(g, dx, dy, dz);
     }
+    const double r = sqrt((double)dx * dx + (double)dy * dy + (double)dz * dz);
+    acc -= (double)x[i].w * (double)x[j].w * erf(screen * r) / r;
+  }
   __shared__ double red[32];
   acc = warp_sum(acc);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
@@ -761,7 +792,8 @@ __global__ void k_selfreal(FrameArgs a, int first, double screen, const float4* 
 
 void launch_selfreal(const FrameArgs& a, const DeviceState& d, int first, int count, double screen, cudaStream_t s) {
   if (count <= 0) return;
-  k_selfreal<<<count, 128, 0, s>>>(a, first, screen, d.tgt_n, d.selfreal);
+  const int threads = std::min(kSelfThreads, std::max(32, (a.nsite * (a.nsite - 1) / 2 + 31) / 32 * 32));
+  k_selfreal<<<count, threads, 0, s>>>(a, first, screen, d.tgt_n, d.selfreal);
 }
 
 // ---------------------------------------------------------------------------
@@ -1707,9 +1739,13 @@ void launch_gather(const FrameArgs& a, const DeviceState& d, int base, int bb, i
 // :917-937), written out as that target's count row.
 // ---------------------------------------------------------------------------
 constexpr int kBinThreads = 256;
+// Few targets (a solution frame has one): wider CTAs, as there are no others to hide a CTA's latency.
+// One target of 4096 molecules: 125 us with 256 threads and a shared FP64 atomic a molecule for the
+// species sums, 16 us with 1024 and the sums kept per thread; below one CTA an SM.
+constexpr int kBinWide = 1024, kBinWideTargets = 148;
 constexpr int kMaxSpecSmem = 128;
 
-__global__ void __launch_bounds__(kBinThreads) k_bin(BinArgs ba, int bb, int slvmax, double* __restrict__ Etot,
+__global__ void __launch_bounds__(kBinWide) k_bin(BinArgs ba, int bb, int slvmax, double* __restrict__ Etot,
     const double* __restrict__ Ereal, bool keep_total,
     const int* __restrict__ molspec, const int* __restrict__ spec_off, const double* __restrict__ uvcrd,
     const int* __restrict__ uvsoft, const int* __restrict__ tgt_mol, const int* __restrict__ skip,
@@ -1742,11 +1778,16 @@ __global__ void __launch_bounds__(kBinThreads) k_bin(BinArgs ba, int bb, int slv
   // to shared memory when the species changes: one atomic pair per run instead of per molecule
   int run_sp = 0;
   float run_min = FLT_MAX, run_max = -FLT_MAX;
+  // solution: the species' energy sums; one species' sum is the target's total, below
+  const bool sums = ba.slttype == ERMOD_SLT_SOLN && ba.numslv > 1;
+  double run_sum = 0.0;
   auto flush_run = [&]() {
     if (run_sp > 0 && run_sp < kMaxSpecSmem) {
       atomic_min_f(&smin[run_sp], run_min);
       atomic_max_f(&smax[run_sp], run_max);
+      if (sums) atomicAdd(&sfl[run_sp], run_sum);
     }
+    run_sum = 0.0;
     run_min = FLT_MAX;
     run_max = -FLT_MAX;
   };
@@ -1782,7 +1823,7 @@ __global__ void __launch_bounds__(kBinThreads) k_bin(BinArgs ba, int bb, int slv
       }
       run_min = fminf(run_min, ef);
       run_max = fmaxf(run_max, ef);
-      if (ba.slttype == ERMOD_SLT_SOLN) atomicAdd(&sfl[pti], e);
+      run_sum += e;
     } else {
       atomic_min_f(&minuv[pti], ef);
       atomic_max_f(&maxuv[pti], ef);
@@ -1798,12 +1839,15 @@ __global__ void __launch_bounds__(kBinThreads) k_bin(BinArgs ba, int bb, int slv
   if (threadIdx.x < 32) {
     double v = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0;
     v = warp_sum(v);
-    if (threadIdx.x == 0) etot[cnt] = v;
+    if (threadIdx.x == 0) {
+      etot[cnt] = v;
+      if (ba.slttype == ERMOD_SLT_SOLN && ba.numslv == 1) flceng[(size_t)cnt] = v;
+    }
   }
   for (int i = threadIdx.x + 1; i < kMaxSpecSmem && i <= ba.numslv; i += blockDim.x) {
     if (smin[i] != FLT_MAX) atomic_min_f(&minuv[i], smin[i]);
     if (smax[i] != -FLT_MAX) atomic_max_f(&maxuv[i], smax[i]);
-    if (ba.slttype == ERMOD_SLT_SOLN) flceng[(size_t)cnt * ba.numslv + i - 1] = sfl[i];
+    if (sums) flceng[(size_t)cnt * ba.numslv + i - 1] = sfl[i];
   }
 }
 
@@ -1813,7 +1857,7 @@ void launch_bin(const DeviceState& d, const BinArgs& ba, int bb, int nbatch, int
                 cudaStream_t s) {
   if (nbatch <= 0) return;
   // the summed energies go back to Etot only when the per-molecule energies are kept (uvengy)
-  k_bin<<<nbatch, kBinThreads, bin_smem_bytes(ba), s>>>(ba, bb, slvmax, d.Etot, d.E, d.uvengy != nullptr, d.molspec,
+  k_bin<<<nbatch, nbatch < kBinWideTargets ? kBinWide : kBinThreads, bin_smem_bytes(ba), s>>>(ba, bb, slvmax, d.Etot, d.E, d.uvengy != nullptr, d.molspec,
                                                         d.spec_off,
                                                         d.uvcrd,
                                                         d.uvsoft, d.tgt_mol, d.skip, d.counts, d.etot, d.flceng,
