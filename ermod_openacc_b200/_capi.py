@@ -148,6 +148,7 @@ SIGNATURES = {
     "ermod_last_error": (C.c_char_p, [C.c_void_p]),
     "ermod_get_timings": (C.c_int32, [C.c_void_p, _f32p, C.c_int32]),
     "ermod_get_launch_count": (C.c_int64, [C.c_void_p]),
+    "ermod_staging_release": (None, []),
     "ermod_get_paths": (C.c_int32, [C.c_void_p, C.POINTER(C.c_int32), C.POINTER(C.c_int32)]),
     "ermod_batch_create": (C.c_int32, [C.POINTER(C.c_void_p), C.c_int32, C.POINTER(C.c_void_p)]),
     "ermod_batch_engconst": (C.c_int32, [C.c_void_p, C.c_int32, C.POINTER(C.c_float), C.POINTER(C.c_float),

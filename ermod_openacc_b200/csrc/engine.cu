@@ -53,6 +53,7 @@ struct ermod_ctx {
   cudaStream_t st = nullptr;
   cudaStream_t st2 = nullptr;            // real space, beside the PME chain of st
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  cudaEvent_t ev_idle = nullptr;         // orders st's earlier work before a batch's stream
   cudaEvent_t ev[9] = {};
   ermod_params p{};
   // host topology
@@ -79,6 +80,11 @@ struct ermod_ctx {
   float invcell_prev[3] = {0.f, 0.f, 0.f};
   float prevcl[9] = {0};
   bool pme_init = false, usreal_init = false, warn_bin_firsttime = true;
+  std::vector<void*> owned;              // device allocations behind palloc's buffers
+  unsigned char* pool = nullptr;         // rest of its last shared block
+  size_t pool_left = 0;
+  unsigned char* h_block = nullptr;      // pinned: h_frame, h_status, h_acc, h_pin
+  float* h_grown = nullptr;              // pinned: h_pin, once a frame's inputs outgrow h_block
   float* h_pin = nullptr;
   size_t h_pin_bytes = 0;
   std::string err;
@@ -97,6 +103,7 @@ struct ermod_ctx {
   long long graph_launches = 0;
   int* h_frame = nullptr;         // pinned: [0] stnum of the frame being staged
   DevStatus* h_status = nullptr;  // pinned: status word written by the frame
+  double* h_acc = nullptr;        // pinned image of the accumulators' allocation (acc_words)
   // insertion proposal: voxels per side (0: off), uniform mixture weight, network loaded
   int prop_gv = 0, prop_gf = 0;
   float prop_eps = 0.1f;
@@ -120,6 +127,32 @@ cudaError_t dalloc(T** p, size_t n) {
   return cudaMalloc((void**)p, n * sizeof(T));
 }
 
+// A buffer of the context's whole life.  Those of at most kPoolMax share blocks of kPoolBlock: a
+// context has some sixty, and an allocation costs about as much for a byte as for a megabyte.
+constexpr size_t kPoolMax = (size_t)1 << 20, kPoolBlock = (size_t)4 << 20;
+
+template <class T>
+cudaError_t palloc(ermod_ctx* c, T** p, size_t n) {
+  const size_t bytes = (std::max<size_t>(n, 1) * sizeof(T) + 255) / 256 * 256;
+  if (bytes <= kPoolMax) {
+    if (c->pool_left < bytes) {
+      unsigned char* q = nullptr;
+      const cudaError_t e = cudaMalloc((void**)&q, kPoolBlock);
+      if (e != cudaSuccess) return e;
+      c->owned.push_back(q);
+      c->pool = q;
+      c->pool_left = kPoolBlock;
+    }
+    *p = (T*)c->pool;
+    c->pool += bytes;
+    c->pool_left -= bytes;
+    return cudaSuccess;
+  }
+  const cudaError_t e = cudaMalloc((void**)p, bytes);
+  if (e == cudaSuccess) c->owned.push_back(*p);
+  return e;
+}
+
 template <class T>
 cudaError_t h2d(T* dst, const T* src, size_t n, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
@@ -128,19 +161,10 @@ cudaError_t h2d(T* dst, const T* src, size_t n, cudaStream_t s) {
 
 void free_all(ermod_ctx* c) {
   DeviceState& d = c->d;
-  void* ptrs[] = {d.molbeg, d.molspec, d.molq, d.atom_lj, d.atom_q, d.ljene, d.ljlensq, d.slt_lj, d.slt_q,
-                  d.slt_mass, d.bfcoord, d.uvcrd, d.spec_off, d.uvsoft, d.escrd, d.posraw, d.slvn, d.spl, d.grd,
-                  d.grec, d.mrec, d.sanch, d.gsph, d.anchor, d.cellof, d.cellcount, d.cellstart, d.molsorted, d.ins_conf,
-                  d.insw_in,
-                  d.tgt_raw, d.tgt_n, d.tgt_c, d.tgt_mol, d.selfreal, d.selfrec, d.u0, d.w, d.etot, d.flceng,
-                  d.grid, d.spec, d.phin, d.phi, d.engfac, d.engfacT, d.fft_tw, d.fft_twd, d.sitetab, d.sitestn,
-                  d.splfc,
-                  d.E, d.Etot, d.tgtq, d.twt, d.sbin, d.gacc,
-                  d.boxinfo, d.partial, d.done, d.uvengy, d.counts, d.edens, d.edens_part, d.ecorr, d.eself,
-                  d.slnuv, d.minuv, d.maxuv, d.scal, d.status, d.frame_i, d.dens, d.feat, d.mlp_f, d.mlp_b,
-                  d.vact, d.vlogit, d.vcdf, d.vq, d.ins_voxel, d.ins_feat, d.host_atom, d.host_mass, d.aggcen,
-                  d.atom_mass, d.skip, d.ref_atom, d.ref_host, d.ref_host_w, d.ref_slt, d.ref_slt_w, d.ref_bf,
-                  c->tc_work};
+  for (void* p : c->owned) cudaFree(p);
+  // what set_refstructure, proposal_config and get_insertion_samples allocate
+  void* ptrs[] = {d.dens, d.feat, d.mlp_f, d.mlp_b, d.vact, d.vlogit, d.vcdf, d.vq, d.ins_voxel, d.ins_feat,
+                  d.ref_atom, d.ref_host, d.ref_host_w, d.ref_slt, d.ref_slt_w, d.ref_bf};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (c->plans) {
@@ -151,12 +175,12 @@ void free_all(ermod_ctx* c) {
     if (e) cudaEventDestroy(e);
   for (auto& e : c->pev)
     if (e) cudaEventDestroy(e);
-  if (c->h_pin) cudaFreeHost(c->h_pin);
-  if (c->h_frame) cudaFreeHost(c->h_frame);
-  if (c->h_status) cudaFreeHost(c->h_status);
+  if (c->h_grown) cudaFreeHost(c->h_grown);
+  if (c->h_block) cudaFreeHost(c->h_block);
   if (c->gexec) cudaGraphExecDestroy(c->gexec);
   if (c->ev_fork) cudaEventDestroy(c->ev_fork);
   if (c->ev_join) cudaEventDestroy(c->ev_join);
+  if (c->ev_idle) cudaEventDestroy(c->ev_idle);
   if (c->st2) cudaStreamDestroy(c->st2);
   if (c->st) cudaStreamDestroy(c->st);
 }
@@ -192,6 +216,11 @@ void spline_axis(int K, int order, double* out) {
     }
     out[rci] = re * re + im * im;
   }
+}
+
+// 8-byte words of the accumulators' allocation (DeviceState::edens .. maxuv)
+size_t acc_words(const ermod_ctx* c) {
+  return (size_t)c->ermax + std::max(1, c->esmax) + c->numslv + 8 + (size_t)(c->numslv + 1);
 }
 
 int set_error(ermod_ctx* c, int code, const char* name) {
@@ -419,26 +448,27 @@ int32_t ermod_create(ermod_ctx** out, int32_t device, const ermod_params* prm, c
   }
   CK(cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming));
   CK(cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming));
+  CK(cudaEventCreateWithFlags(&ctx->ev_idle, cudaEventDisableTiming));
   for (auto& e : ctx->ev) CK(cudaEventCreate(&e));
   DeviceState& d = ctx->d;
   const size_t NA = ctx->natoms, SM = ctx->slvmax, MD = ctx->maxdst, S = ctx->s;
   const int order = pme ? p.splodr : 1;
-  CK(dalloc(&d.molbeg, SM + 1)); CK(dalloc(&d.molspec, SM)); CK(dalloc(&d.molq, SM));
-  CK(dalloc(&d.atom_lj, NA)); CK(dalloc(&d.atom_q, NA));
-  CK(dalloc(&d.ljene, (size_t)ctx->ljtype_max * ctx->ljtype_max));
-  CK(dalloc(&d.ljlensq, (size_t)ctx->ljtype_max * ctx->ljtype_max));
-  CK(dalloc(&d.slt_lj, S)); CK(dalloc(&d.slt_q, S)); CK(dalloc(&d.slt_mass, S)); CK(dalloc(&d.bfcoord, 3 * S));
-  CK(dalloc(&d.uvcrd, ctx->ermax)); CK(dalloc(&d.spec_off, ctx->numslv + 1)); CK(dalloc(&d.uvsoft, ctx->numslv));
-  CK(dalloc(&d.escrd, std::max(1, ctx->esmax)));
-  CK(dalloc(&d.posraw, 3 * NA)); CK(dalloc(&d.slvn, NA)); CK(dalloc(&d.spl, NA * 3 * order)); CK(dalloc(&d.grd, NA));
-  if (pme && gather_rec_ok(order, K1, K2, K3)) CK(dalloc(&d.grec, NA * kRecWords));
-  CK(dalloc(&d.mrec, SM)); CK(dalloc(&d.sanch, SM)); CK(dalloc(&d.gsph, (SM + 31) / 32));
-  CK(dalloc(&d.anchor, SM)); CK(dalloc(&d.cellof, SM)); CK(dalloc(&d.cellcount, ctx->ncell_cap));
-  CK(dalloc(&d.cellstart, ctx->ncell_cap + 1)); CK(dalloc(&d.molsorted, SM));
-  CK(dalloc(&d.ins_conf, 3 * S * MD)); CK(dalloc(&d.insw_in, MD));
-  CK(dalloc(&d.tgt_raw, MD * S)); CK(dalloc(&d.tgt_n, MD * S)); CK(dalloc(&d.tgt_c, MD)); CK(dalloc(&d.tgt_mol, MD));
-  CK(dalloc(&d.selfreal, MD)); CK(dalloc(&d.selfrec, MD)); CK(dalloc(&d.u0, MD)); CK(dalloc(&d.w, MD));
-  CK(dalloc(&d.etot, MD)); CK(dalloc(&d.flceng, MD * ctx->numslv));
+  CK(palloc(ctx, &d.molbeg, SM + 1)); CK(palloc(ctx, &d.molspec, SM)); CK(palloc(ctx, &d.molq, SM));
+  CK(palloc(ctx, &d.atom_lj, NA)); CK(palloc(ctx, &d.atom_q, NA));
+  CK(palloc(ctx, &d.ljene, (size_t)ctx->ljtype_max * ctx->ljtype_max));
+  CK(palloc(ctx, &d.ljlensq, (size_t)ctx->ljtype_max * ctx->ljtype_max));
+  CK(palloc(ctx, &d.slt_lj, S)); CK(palloc(ctx, &d.slt_q, S)); CK(palloc(ctx, &d.slt_mass, S)); CK(palloc(ctx, &d.bfcoord, 3 * S));
+  CK(palloc(ctx, &d.uvcrd, ctx->ermax)); CK(palloc(ctx, &d.spec_off, ctx->numslv + 1)); CK(palloc(ctx, &d.uvsoft, ctx->numslv));
+  CK(palloc(ctx, &d.escrd, std::max(1, ctx->esmax)));
+  CK(palloc(ctx, &d.posraw, 3 * NA)); CK(palloc(ctx, &d.slvn, NA)); CK(palloc(ctx, &d.spl, NA * 3 * order)); CK(palloc(ctx, &d.grd, NA));
+  if (pme && gather_rec_ok(order, K1, K2, K3)) CK(palloc(ctx, &d.grec, NA * kRecWords));
+  CK(palloc(ctx, &d.mrec, SM)); CK(palloc(ctx, &d.sanch, SM)); CK(palloc(ctx, &d.gsph, (SM + 31) / 32));
+  CK(palloc(ctx, &d.anchor, SM)); CK(palloc(ctx, &d.cellof, SM)); CK(palloc(ctx, &d.cellcount, ctx->ncell_cap));
+  CK(palloc(ctx, &d.cellstart, ctx->ncell_cap + 1)); CK(palloc(ctx, &d.molsorted, SM));
+  CK(palloc(ctx, &d.ins_conf, 3 * S * MD)); CK(palloc(ctx, &d.insw_in, MD));
+  CK(palloc(ctx, &d.tgt_raw, MD * S)); CK(palloc(ctx, &d.tgt_n, MD * S)); CK(palloc(ctx, &d.tgt_c, MD)); CK(palloc(ctx, &d.tgt_mol, MD));
+  CK(palloc(ctx, &d.selfreal, MD)); CK(palloc(ctx, &d.selfrec, MD)); CK(palloc(ctx, &d.u0, MD)); CK(palloc(ctx, &d.w, MD));
+  CK(palloc(ctx, &d.etot, MD)); CK(palloc(ctx, &d.flceng, MD * ctx->numslv));
   const size_t KK = (size_t)K1 * K2 * K3, KH = (size_t)K3 * K2 * Kh1;
   // PME solve path (spectrum_path): the fused solve where the mesh allows it
   FrameArgs fa{};
@@ -457,51 +487,61 @@ int32_t ermod_create(ermod_ctx** out, int32_t device, const ermod_params* prm, c
   if (p.spectrum_path == 0) ctx->spath = fused_ok ? (ctx->s <= direct_auto ? 2 : 3) : 1;
   else ctx->spath = p.spectrum_path;
   if (pme) {
-    CK(dalloc(&d.spec, (size_t)ctx->chunk * KH));
-    CK(dalloc(&d.phi, (size_t)ctx->chunk * K3 * K2 * 2 * ((K1 + 1) / 2)));   // n1 pairs, see DeviceState::phi
-    CK(dalloc(&d.engfac, KH)); CK(dalloc(&d.splfc, K1 + K2 + K3));
+    CK(palloc(ctx, &d.spec, (size_t)ctx->chunk * KH));
+    CK(palloc(ctx, &d.phi, (size_t)ctx->chunk * K3 * K2 * 2 * ((K1 + 1) / 2)));   // n1 pairs, see DeviceState::phi
+    CK(palloc(ctx, &d.engfac, KH)); CK(palloc(ctx, &d.splfc, K1 + K2 + K3));
     if (ctx->spath == 1) {
-      CK(dalloc(&d.grid, (size_t)ctx->chunk * KK));
+      CK(palloc(ctx, &d.grid, (size_t)ctx->chunk * KK));
       CK(cudaMemsetAsync(d.grid, 0, sizeof(float) * ctx->chunk * KK, ctx->st));  // kept zero outside the boxes
-      CK(dalloc(&d.phin, (size_t)ctx->chunk * KK));
+      CK(palloc(ctx, &d.phin, (size_t)ctx->chunk * KK));
     } else {
-      CK(dalloc(&d.engfacT, KH));
+      CK(palloc(ctx, &d.engfacT, KH));
       std::vector<float2> tw;
       std::vector<double2> twd;
       fused_twiddles(K1, K2, K3, tw, twd);
-      CK(dalloc(&d.fft_tw, tw.size()));
-      CK(dalloc(&d.fft_twd, twd.size()));
-      CK(dalloc(&d.sitetab, fused_sitetab_elems(fa, ctx->batch, ctx->spath == 2)));
-      if (ctx->spath == 3) CK(dalloc(&d.sitestn, fused_sitestn_elems(fa, ctx->batch)));
+      CK(palloc(ctx, &d.fft_tw, tw.size()));
+      CK(palloc(ctx, &d.fft_twd, twd.size()));
+      CK(palloc(ctx, &d.sitetab, fused_sitetab_elems(fa, ctx->batch, ctx->spath == 2)));
+      if (ctx->spath == 3) CK(palloc(ctx, &d.sitestn, fused_sitestn_elems(fa, ctx->batch)));
       CK(cudaMemcpyAsync(d.fft_tw, tw.data(), sizeof(float2) * tw.size(), cudaMemcpyHostToDevice, ctx->st));
       CK(cudaMemcpyAsync(d.fft_twd, twd.data(), sizeof(double2) * twd.size(), cudaMemcpyHostToDevice, ctx->st));
       CK(cudaStreamSynchronize(ctx->st));
       if (setup_fused(fa) != 0) return bad(ERMOD_ERR_CUDA, "pme_smem");
     }
   }
-  CK(dalloc(&d.E, SM * ctx->batch));
-  CK(dalloc(&d.Etot, SM * ctx->batch));
-  CK(dalloc(&d.tgtq, MD));
-  CK(dalloc(&d.twt, MD));
-  CK(dalloc(&d.sbin, MD));
+  CK(palloc(ctx, &d.E, SM * ctx->batch));
+  CK(palloc(ctx, &d.Etot, SM * ctx->batch));
+  CK(palloc(ctx, &d.tgtq, MD));
+  CK(palloc(ctx, &d.twt, MD));
+  CK(palloc(ctx, &d.sbin, MD));
   if (pme) {
-    if (ctx->spath == 1) CK(dalloc(&d.gacc, (size_t)ctx->chunk * KK));
-    CK(dalloc(&d.boxinfo, 2 * (size_t)ctx->chunk));
-    CK(dalloc(&d.partial, (size_t)ctx->chunk * std::max(kInflBlocks, Kh1)));
-    CK(dalloc(&d.done, (size_t)ctx->chunk));
+    if (ctx->spath == 1) CK(palloc(ctx, &d.gacc, (size_t)ctx->chunk * KK));
+    CK(palloc(ctx, &d.boxinfo, 2 * (size_t)ctx->chunk));
+    CK(palloc(ctx, &d.partial, (size_t)ctx->chunk * std::max(kInflBlocks, Kh1)));
+    CK(palloc(ctx, &d.done, (size_t)ctx->chunk));
     CK(cudaMemsetAsync(d.done, 0, sizeof(unsigned int) * ctx->chunk, ctx->st));
     if (setup_spread_smem() != 0) return bad(ERMOD_ERR_CUDA, "spr_smem");
   }
-  if (p.keep_uvengy) CK(dalloc(&d.uvengy, MD * SM));
-  CK(dalloc(&d.counts, (size_t)ctx->batch * ctx->ermax_pad));
-  CK(dalloc(&d.edens, ctx->ermax));
-  CK(dalloc(&d.edens_part, (size_t)kEdensSlices * ctx->ermax));
-  if (p.corrcal) CK(dalloc(&d.ecorr, (size_t)ctx->ermax * ctx->ermax));
-  CK(dalloc(&d.eself, std::max(1, ctx->esmax))); CK(dalloc(&d.slnuv, ctx->numslv));
-  CK(dalloc(&d.minuv, ctx->numslv + 1)); CK(dalloc(&d.maxuv, ctx->numslv + 1));
-  CK(dalloc(&d.scal, 8)); CK(dalloc(&d.status, 1)); CK(dalloc(&d.frame_i, 4));
-  CK(cudaMallocHost((void**)&ctx->h_frame, 4 * sizeof(int)));
-  CK(cudaMallocHost((void**)&ctx->h_status, sizeof(DevStatus)));
+  if (p.keep_uvengy) CK(palloc(ctx, &d.uvengy, MD * SM));
+  CK(palloc(ctx, &d.counts, (size_t)ctx->batch * ctx->ermax_pad));
+  CK(palloc(ctx, &d.edens, acc_words(ctx)));
+  d.eself = d.edens + ctx->ermax;
+  d.slnuv = d.eself + std::max(1, ctx->esmax);
+  d.scal = d.slnuv + ctx->numslv;
+  d.minuv = (float*)(d.scal + 8);
+  d.maxuv = d.minuv + ctx->numslv + 1;
+  CK(palloc(ctx, &d.edens_part, (size_t)kEdensSlices * ctx->ermax));
+  if (p.corrcal) CK(palloc(ctx, &d.ecorr, (size_t)ctx->ermax * ctx->ermax));
+  CK(palloc(ctx, &d.status, 1)); CK(palloc(ctx, &d.frame_i, 4));
+  {   // pinned: the staged scalars, the status word, the accumulators' image and a frame's inputs
+    const size_t acc = sizeof(double) * acc_words(ctx), in = sizeof(float) * (3 * NA + MD);
+    CK(cudaMallocHost((void**)&ctx->h_block, 128 + acc + in));
+    ctx->h_frame = (int*)ctx->h_block;
+    ctx->h_status = (DevStatus*)(ctx->h_block + 64);
+    ctx->h_acc = (double*)(ctx->h_block + 128);
+    ctx->h_pin = (float*)(ctx->h_block + 128 + acc);
+    ctx->h_pin_bytes = in;
+  }
   if (p.graph_mode < 0 || p.graph_mode > 1 || p.stage_timing < 0 || p.stage_timing > 1) return bad(ERMOD_ERR_ARG, "opt_arg");
   // static uploads
   cudaStream_t st = ctx->st;
@@ -513,7 +553,7 @@ int32_t ermod_create(ermod_ctx** out, int32_t device, const ermod_params* prm, c
   CK(h2d(d.slt_lj, slt_lj.data(), S, st)); CK(h2d(d.slt_q, slt_q.data(), S, st));
   CK(h2d(d.slt_mass, slt_m.data(), S, st));
   if (ctx->nhost > 0) {
-    CK(dalloc(&d.host_atom, ctx->nhost)); CK(dalloc(&d.host_mass, ctx->nhost)); CK(dalloc(&d.aggcen, 3));
+    CK(palloc(ctx, &d.host_atom, ctx->nhost)); CK(palloc(ctx, &d.host_mass, ctx->nhost)); CK(palloc(ctx, &d.aggcen, 3));
     CK(h2d(d.host_atom, host_atom.data(), ctx->nhost, st));
     CK(h2d(d.host_mass, host_mass.data(), ctx->nhost, st));
     if (!refs) {   // solute centres of mass for check_mol_configuration, and its verdicts
@@ -523,13 +563,13 @@ int32_t ermod_create(ermod_ctx** out, int32_t device, const ermod_params* prm, c
         const int i = ctx->tagpt[k];
         for (int j = 0; j < ctx->numsite[i]; ++j) am.push_back(ctx->mass[ctx->molbeg_all[i] + j]);
       }
-      CK(dalloc(&d.atom_mass, NA));
+      CK(palloc(ctx, &d.atom_mass, NA));
       CK(h2d(d.atom_mass, am.data(), NA, st));
     }
   }
   // soln: the verdicts of check_mol_configuration (sphere / slab around the aggregate, RMSD to RefInfo)
   if (!refs && (ctx->nhost > 0 || p.insposition == ERMOD_INSPOS_RMSD || p.insstructure == ERMOD_INSSTR_RMSD))
-    CK(dalloc(&d.skip, MD));
+    CK(palloc(ctx, &d.skip, MD));
   std::vector<float> bf(3 * S, 0.0f);
   if (t->bfcoord) std::memcpy(bf.data(), t->bfcoord, sizeof(float) * 3 * S);
   CK(h2d(d.bfcoord, bf.data(), 3 * S, st));
@@ -597,7 +637,7 @@ int32_t ermod_create(ermod_ctx** out, int32_t device, const ermod_params* prm, c
   ctx->use_tc = (p.corrcal && ecorr_tc_available() && p.ecorr_path == 0) ? 1 : 0;
   if (ctx->use_tc) {
     ctx->tc_work_bytes = ecorr_tc_workspace(ctx->batch, ctx->ermax);
-    CK(cudaMalloc(&ctx->tc_work, ctx->tc_work_bytes));
+    CK(palloc(ctx, (unsigned char**)&ctx->tc_work, ctx->tc_work_bytes));
   }
   const int rc = ermod_engclear(ctx);
   if (rc != ERMOD_OK) return rc;
@@ -654,13 +694,10 @@ int32_t ermod_engclear(ermod_ctx* ctx) {
   CK(cudaSetDevice(ctx->device));
   DeviceState& d = ctx->d;
   cudaStream_t st = ctx->st;
-  CK(cudaMemsetAsync(d.edens, 0, sizeof(double) * ctx->ermax, st));
+  // edens, eself, slnuv and avslf, engnorm, engsmpl (scal[0..2]); voffset and the self-energy reuse
+  // persist.  In stream order: the context's next frame or read-back runs on st, a batch waits for it.
+  CK(cudaMemsetAsync(d.edens, 0, (size_t)((char*)(d.scal + 3) - (char*)d.edens), st));
   if (d.ecorr) CK(cudaMemsetAsync(d.ecorr, 0, sizeof(double) * ctx->ermax * ctx->ermax, st));
-  CK(cudaMemsetAsync(d.eself, 0, sizeof(double) * std::max(1, ctx->esmax), st));
-  CK(cudaMemsetAsync(d.slnuv, 0, sizeof(double) * ctx->numslv, st));
-  // avslf, engnorm, engsmpl (scal[0..2]); voffset and the self-energy reuse persist
-  CK(cudaMemsetAsync(d.scal, 0, sizeof(double) * 3, st));
-  CK(cudaStreamSynchronize(st));
   return ERMOD_OK;
 }
 
@@ -1210,9 +1247,12 @@ static int stage_host_inputs(ermod_ctx* ctx, const float* sitepos, const float* 
   const size_t nconf = (refs && ins_conf) ? 3 * (size_t)ctx->s * ctx->maxdst : 0;
   const size_t need = sizeof(float) * (npos + nconf + ctx->maxdst);
   if (ctx->h_pin_bytes < need) {
-    if (ctx->h_pin) cudaFreeHost(ctx->h_pin);
-    ctx->h_pin = nullptr;
-    CK(cudaMallocHost((void**)&ctx->h_pin, need));
+    // the new buffer first: should it fail, the context keeps the old one
+    float* grown = nullptr;
+    CK(cudaMallocHost((void**)&grown, need));
+    CK(cudaStreamSynchronize(ctx->st));   // the old one may still feed the previous frame's copies
+    if (ctx->h_grown) cudaFreeHost(ctx->h_grown);
+    ctx->h_pin = ctx->h_grown = grown;
     ctx->h_pin_bytes = need;
   }
   CK(cudaStreamSynchronize(ctx->st));   // the staging buffer may still feed the previous frame's copies
@@ -1347,9 +1387,13 @@ static int batch_run(ermod_batch* b, int stnum, const float* cell, float wsys) {
     if (rc != ERMOD_OK) return fail_member(i, rc);
     if (ctx->real_threads == 0) tuned = false;
   }
-  // stage every member's inputs on the batch stream, ahead of the graph
+  // stage every member's inputs on the batch stream, ahead of the graph and behind what the member's
+  // own stream still holds (engclear)
   for (int i = 0; i < n; ++i) {
     ermod_ctx* ctx = b->m[i];
+    if (cudaEventRecord(ctx->ev_idle, ctx->st) != cudaSuccess ||
+        cudaStreamWaitEvent(b->st, ctx->ev_idle, 0) != cudaSuccess)
+      return ERMOD_ERR_CUDA;
     if (cudaMemcpyAsync(ctx->d.posraw, b->d_pos, sizeof(float) * b->npos, cudaMemcpyDeviceToDevice, b->st) !=
         cudaSuccess)
       return ERMOD_ERR_CUDA;
@@ -1460,39 +1504,55 @@ void ermod_batch_destroy(ermod_batch* b) {
   delete b;
 }
 
-int32_t ermod_fetch_accum(ermod_ctx* ctx, ermod_accum* o) {
-  if (!ctx || !o) return ERMOD_ERR_ARG;
+}  // extern "C"
+
+// Below this the correlation matrix is copied directly: threads and slots cost tens of microseconds.
+constexpr size_t kStagedBytes = (size_t)1 << 20;
+
+// The raw accumulators into *o but for ecorr, whose values are divided by engnorm when `normalise`.
+static int read_accum(ermod_ctx* ctx, ermod_accum* o, bool normalise) {
   CK(cudaSetDevice(ctx->device));
-  CK(cudaStreamSynchronize(ctx->st));
   const DeviceState& d = ctx->d;
-  if (o->edens) CK(cudaMemcpy(o->edens, d.edens, sizeof(double) * ctx->ermax, cudaMemcpyDeviceToHost));
-  if (o->ecorr && d.ecorr)
-    CK(cudaMemcpy(o->ecorr, d.ecorr, sizeof(double) * ctx->ermax * ctx->ermax, cudaMemcpyDeviceToHost));
-  if (o->eself && ctx->p.selfcal) CK(cudaMemcpy(o->eself, d.eself, sizeof(double) * ctx->esmax, cudaMemcpyDeviceToHost));
-  if (o->slnuv) {
-    std::vector<double> s(ctx->numslv);
-    CK(cudaMemcpy(s.data(), d.slnuv, sizeof(double) * ctx->numslv, cudaMemcpyDeviceToHost));
-    for (int i = 0; i < ctx->numslv; ++i) o->slnuv[i] = (float)s[i];
-  }
-  if (o->minuv) CK(cudaMemcpy(o->minuv, d.minuv, sizeof(float) * (ctx->numslv + 1), cudaMemcpyDeviceToHost));
-  if (o->maxuv) CK(cudaMemcpy(o->maxuv, d.maxuv, sizeof(float) * (ctx->numslv + 1), cudaMemcpyDeviceToHost));
-  double sc[8];
-  CK(cudaMemcpy(sc, d.scal, sizeof(sc), cudaMemcpyDeviceToHost));
+  CK(cudaMemcpyAsync(ctx->h_acc, d.edens, sizeof(double) * acc_words(ctx), cudaMemcpyDeviceToHost, ctx->st));
+  CK(cudaStreamSynchronize(ctx->st));
+  auto host = [&](const void* p) { return (const unsigned char*)ctx->h_acc + ((const char*)p - (const char*)d.edens); };
+  if (o->edens) std::memcpy(o->edens, host(d.edens), sizeof(double) * ctx->ermax);
+  if (o->eself && ctx->p.selfcal) std::memcpy(o->eself, host(d.eself), sizeof(double) * ctx->esmax);
+  if (o->slnuv)
+    for (int i = 0; i < ctx->numslv; ++i) o->slnuv[i] = (float)((const double*)host(d.slnuv))[i];
+  if (o->minuv) std::memcpy(o->minuv, host(d.minuv), sizeof(float) * (ctx->numslv + 1));
+  if (o->maxuv) std::memcpy(o->maxuv, host(d.maxuv), sizeof(float) * (ctx->numslv + 1));
+  const double* sc = (const double*)host(d.scal);
   o->avslf = sc[0];
   o->engnorm = sc[1];
   o->engsmpl = sc[2];
   o->voffset = sc[3];
   o->voffset_initialized = sc[4] != 0.0;
+  if (o->ecorr && d.ecorr) {
+    const size_t bytes = sizeof(double) * ctx->ermax * ctx->ermax;
+    // a zero norm (no insertion kept) divides on the host, where 0 / 0 is what it was
+    const double q = normalise && bytes > kStagedBytes ? o->engnorm : 0.0;
+    if (bytes > kStagedBytes) CK(staged_to_host(o->ecorr, d.ecorr, bytes, q, ctx->st));
+    else CK(cudaMemcpy(o->ecorr, d.ecorr, bytes, cudaMemcpyDeviceToHost));
+    if (normalise && q == 0.0)
+      for (size_t i = 0; i < (size_t)ctx->ermax * ctx->ermax; ++i) o->ecorr[i] /= o->engnorm;
+  }
   return ERMOD_OK;
+}
+
+extern "C" {
+
+int32_t ermod_fetch_accum(ermod_ctx* ctx, ermod_accum* o) {
+  if (!ctx || !o) return ERMOD_ERR_ARG;
+  return read_accum(ctx, o, false);
 }
 
 int32_t ermod_engstore(ermod_ctx* ctx, ermod_accum* o, double* avediv) {
   if (!ctx || !o) return ERMOD_ERR_ARG;
-  const int rc = ermod_fetch_accum(ctx, o);
+  const int rc = read_accum(ctx, o, true);   // ecorr comes back divided by engnorm
   if (rc != ERMOD_OK) return rc;
   const double nrm = o->engnorm;  // engproc.F90:609-628
   if (o->edens) for (int i = 0; i < ctx->ermax; ++i) o->edens[i] /= nrm;
-  if (o->ecorr && ctx->d.ecorr) for (size_t i = 0; i < (size_t)ctx->ermax * ctx->ermax; ++i) o->ecorr[i] /= nrm;
   if (o->eself && ctx->p.selfcal) for (int i = 0; i < ctx->esmax; ++i) o->eself[i] /= nrm;
   // soln: aveuv(division, :) = slnuv / engnorm (engproc.F90:622), returned in slnuv
   if (o->slnuv && ctx->p.slttype == ERMOD_SLT_SOLN)

@@ -172,15 +172,16 @@ struct DeviceState {
   unsigned int* done = nullptr; // [chunk] block counters of the self-energy reduction
   double* uvengy = nullptr;  // [maxdst*slvmax] kept when requested
   uint32_t* counts = nullptr;// [batch*ermax_pad]
-  // accumulators
+  // accumulators: one allocation, in this order (edens .. scal[2] are cleared together, all are read back together),
+  // but for ecorr
   double* edens = nullptr;   // [ermax]
-  double* edens_part = nullptr; // [kEdensSlices*ermax] partial sums (NULL: one-pass edens kernel)
-  double* ecorr = nullptr;   // [ermax*ermax]
-  double* eself = nullptr;   // [esmax]
+  double* eself = nullptr;   // [max(1, esmax)]
   double* slnuv = nullptr;   // [numslv]
+  double* scal = nullptr;    // [8]: avslf, engnorm, engsmpl, voffset, voffset_init, usreal, usreal_init
   float* minuv = nullptr;    // [numslv+1]
   float* maxuv = nullptr;    // [numslv+1]
-  double* scal = nullptr;    // [8]: avslf, engnorm, engsmpl, voffset, voffset_init, usreal, usreal_init
+  double* ecorr = nullptr;   // [ermax*ermax]
+  double* edens_part = nullptr; // [kEdensSlices*ermax] partial sums (NULL: one-pass edens kernel)
   DevStatus* status = nullptr;
   int* frame_i = nullptr;    // [4] per-frame scalars staged before the frame: [0] stnum
   // insertion proposal (refs mode)
@@ -207,6 +208,11 @@ struct DeviceState {
   int* ins_voxel = nullptr;  // [maxdst] voxel of each insertion
   float* ins_feat = nullptr; // [maxdst][64] features of each insertion's voxel (training data, on request)
 };
+
+// Copies of pageable host memory through the pinned ring (staging.cu); they return when the bytes
+// have moved.  `q` != 0: the FP64 values divided by it.
+cudaError_t staged_to_host(void* dst, const void* src, size_t bytes, double q, cudaStream_t s);
+cudaError_t staged_to_device(void* dst, const void* src, size_t bytes, cudaStream_t s);
 
 // ---- launchers (kernels.cu) -------------------------------------------
 void launch_prepare_solvent(const FrameArgs& a, const DeviceState& d, cudaStream_t s);

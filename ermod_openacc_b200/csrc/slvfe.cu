@@ -38,6 +38,10 @@
 
 #include "../../include/ermod_slvfe.h"
 
+namespace erm {
+cudaError_t staged_to_device(void* dst, const void* src, size_t bytes, cudaStream_t s);   // staging.cu
+}
+
 namespace {
 
 constexpr int kTile = 32;
@@ -896,7 +900,7 @@ extern "C" int32_t ermod_slvfe_delta_mu_layout(int32_t device, int32_t n0, int32
   ok = ok && cudaMemcpyAsync(arena + o_rng, rng.data(), sizeof(int4) * n, cudaMemcpyHostToDevice, st) == cudaSuccess;
   ok = ok && cudaMemcpyAsync(ip(o_off), off.data(), 4 * off.size(), cudaMemcpyHostToDevice, st) == cudaSuccess;
   ok = ok && cudaMemsetAsync(d_out, 0, 8 * (size_t)(nsp + 2) + 8, st) == cudaSuccess;
-  ok = ok && cudaMemcpyAsync(d_chi0, chi_ref, 8 * nn0, cudaMemcpyHostToDevice, st) == cudaSuccess;
+  ok = ok && erm::staged_to_device(d_chi0, chi_ref, 8 * nn0, st) == cudaSuccess;
   SlvArgs a{n, nsp, kT, n0, d_rd0, d_rr0, d_rd, d_rr, d_crd, ip(o_spec), dp(o_rho), dp(o_rho0), dp(o_nm), dp(o_om),
             ip(o_both), dp(o_harm), dp(o_reg), d_st, ip(o_off), opts->functional, opts->et};
   const int4* d_rng = (const int4*)(arena + o_rng);

@@ -108,7 +108,7 @@ class Engine:
 
     def _accum_struct(self, ecorr: bool = True):
         ed = np.zeros(self.ermax)
-        ec = np.zeros(self.ermax * self.ermax) if self.params["corrcal"] and ecorr else None
+        ec = np.empty(self.ermax * self.ermax) if self.params["corrcal"] and ecorr else None
         es = np.zeros(self.esmax) if self.params["selfcal"] else None
         sl = np.zeros(self.numslv, dtype=np.float32)
         mn = np.zeros(self.numslv + 1, dtype=np.float32)

@@ -321,6 +321,11 @@ int32_t ermod_get_timings(const ermod_ctx* ctx, float* ms, int32_t n);
  * reference counterpart). */
 int32_t ermod_get_paths(const ermod_ctx* ctx, int32_t* spectrum_path, int32_t* ecorr_path);
 
+/* Large results and inputs (the correlation matrix of engstore, fetch_accum and slvfe) pass
+ * through one 12 MB ring of pinned memory a process, kept between calls; this frees it.  No
+ * such call may be running. */
+void ermod_staging_release(void);
+
 /* Kernel launches of this library since the context was created, cuFFT's
  * own kernels excluded (no reference counterpart; profiling). */
 int64_t ermod_get_launch_count(const ermod_ctx* ctx);
