@@ -53,6 +53,7 @@ struct ermod_ctx {
   cudaStream_t st = nullptr;
   cudaStream_t st2 = nullptr;            // real space, beside the PME chain of st
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  cudaEvent_t ev_prep = nullptr;         // the frame's solvent preparation, on st2
   cudaEvent_t ev_idle = nullptr;         // orders st's earlier work before a batch's stream
   cudaEvent_t ev[9] = {};
   ermod_params p{};
@@ -83,9 +84,9 @@ struct ermod_ctx {
   std::vector<void*> owned;              // device allocations behind palloc's buffers
   unsigned char* pool = nullptr;         // rest of its last shared block
   size_t pool_left = 0;
-  unsigned char* h_block = nullptr;      // pinned: h_frame, h_status, h_acc, h_pin
-  float* h_grown = nullptr;              // pinned: h_pin, once a frame's inputs outgrow h_block
-  float* h_pin = nullptr;
+  unsigned char* h_block = nullptr;      // pinned: h_status, h_acc, h_pin
+  unsigned char* h_grown = nullptr;      // pinned: h_pin, once a frame's inputs outgrow h_block
+  unsigned char* h_pin = nullptr;        // image of the staged inputs (DeviceState::frame_i on)
   size_t h_pin_bytes = 0;
   std::string err;
   // stage timing: events recorded on the stream between stages, read once per frame
@@ -101,7 +102,6 @@ struct ermod_ctx {
   cudaGraphExec_t gexec = nullptr;
   std::vector<unsigned char> gkey;
   long long graph_launches = 0;
-  int* h_frame = nullptr;         // pinned: [0] stnum of the frame being staged
   DevStatus* h_status = nullptr;  // pinned: status word written by the frame
   double* h_acc = nullptr;        // pinned image of the accumulators' allocation (acc_words)
   // insertion proposal: voxels per side (0: off), uniform mixture weight, network loaded
@@ -181,6 +181,7 @@ void free_all(ermod_ctx* c) {
   if (c->ev_fork) cudaEventDestroy(c->ev_fork);
   if (c->ev_join) cudaEventDestroy(c->ev_join);
   if (c->ev_idle) cudaEventDestroy(c->ev_idle);
+  if (c->ev_prep) cudaEventDestroy(c->ev_prep);
   if (c->st2) cudaStreamDestroy(c->st2);
   if (c->st) cudaStreamDestroy(c->st);
 }
@@ -217,6 +218,15 @@ void spline_axis(int K, int order, double* out) {
     out[rci] = re * re + im * im;
   }
 }
+
+// a frame's staged inputs: 16 bytes of scalars (stnum), insertion weights, coordinates, conformations
+constexpr size_t kInHead = 16;
+size_t in_bytes(const ermod_ctx* c, size_t nconf) {
+  return kInHead + sizeof(float) * ((size_t)c->maxdst + 3 * (size_t)c->natoms + nconf);
+}
+
+// what a frame starts from zero: the status word (64 bytes), etot, selfrec, flceng
+size_t frame_zero_bytes(const ermod_ctx* c) { return 64 + sizeof(double) * (size_t)c->maxdst * (2 + c->numslv); }
 
 // 8-byte words of the accumulators' allocation (DeviceState::edens .. maxuv)
 size_t acc_words(const ermod_ctx* c) {
@@ -449,6 +459,7 @@ int32_t ermod_create(ermod_ctx** out, int32_t device, const ermod_params* prm, c
   CK(cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming));
   CK(cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming));
   CK(cudaEventCreateWithFlags(&ctx->ev_idle, cudaEventDisableTiming));
+  CK(cudaEventCreateWithFlags(&ctx->ev_prep, cudaEventDisableTiming));
   for (auto& e : ctx->ev) CK(cudaEventCreate(&e));
   DeviceState& d = ctx->d;
   const size_t NA = ctx->natoms, SM = ctx->slvmax, MD = ctx->maxdst, S = ctx->s;
@@ -460,15 +471,18 @@ int32_t ermod_create(ermod_ctx** out, int32_t device, const ermod_params* prm, c
   CK(palloc(ctx, &d.slt_lj, S)); CK(palloc(ctx, &d.slt_q, S)); CK(palloc(ctx, &d.slt_mass, S)); CK(palloc(ctx, &d.bfcoord, 3 * S));
   CK(palloc(ctx, &d.uvcrd, ctx->ermax)); CK(palloc(ctx, &d.spec_off, ctx->numslv + 1)); CK(palloc(ctx, &d.uvsoft, ctx->numslv));
   CK(palloc(ctx, &d.escrd, std::max(1, ctx->esmax)));
-  CK(palloc(ctx, &d.posraw, 3 * NA)); CK(palloc(ctx, &d.slvn, NA)); CK(palloc(ctx, &d.spl, NA * 3 * order)); CK(palloc(ctx, &d.grd, NA));
+  // a frame's inputs share an allocation, in the order of the pinned image that feeds them (stage_host_inputs)
+  CK(palloc(ctx, (unsigned char**)&d.frame_i, in_bytes(ctx, refs ? 3 * S * MD : 0)));
+  d.insw_in = (float*)((unsigned char*)d.frame_i + kInHead);
+  d.posraw = d.insw_in + MD;
+  d.ins_conf = d.posraw + 3 * NA;
+  CK(palloc(ctx, &d.slvn, NA)); CK(palloc(ctx, &d.spl, NA * 3 * order)); CK(palloc(ctx, &d.grd, NA));
   if (pme && gather_rec_ok(order, K1, K2, K3)) CK(palloc(ctx, &d.grec, NA * kRecWords));
   CK(palloc(ctx, &d.mrec, SM)); CK(palloc(ctx, &d.sanch, SM)); CK(palloc(ctx, &d.gsph, (SM + 31) / 32));
   CK(palloc(ctx, &d.anchor, SM)); CK(palloc(ctx, &d.cellof, SM)); CK(palloc(ctx, &d.cellcount, ctx->ncell_cap));
   CK(palloc(ctx, &d.cellstart, ctx->ncell_cap + 1)); CK(palloc(ctx, &d.molsorted, SM));
-  CK(palloc(ctx, &d.ins_conf, 3 * S * MD)); CK(palloc(ctx, &d.insw_in, MD));
   CK(palloc(ctx, &d.tgt_raw, MD * S)); CK(palloc(ctx, &d.tgt_n, MD * S)); CK(palloc(ctx, &d.tgt_c, MD)); CK(palloc(ctx, &d.tgt_mol, MD));
-  CK(palloc(ctx, &d.selfreal, MD)); CK(palloc(ctx, &d.selfrec, MD)); CK(palloc(ctx, &d.u0, MD)); CK(palloc(ctx, &d.w, MD));
-  CK(palloc(ctx, &d.etot, MD)); CK(palloc(ctx, &d.flceng, MD * ctx->numslv));
+  CK(palloc(ctx, &d.selfreal, MD)); CK(palloc(ctx, &d.u0, MD)); CK(palloc(ctx, &d.w, MD));
   const size_t KK = (size_t)K1 * K2 * K3, KH = (size_t)K3 * K2 * Kh1;
   // PME solve path (spectrum_path): the fused solve where the mesh allows it
   FrameArgs fa{};
@@ -532,14 +546,18 @@ int32_t ermod_create(ermod_ctx** out, int32_t device, const ermod_params* prm, c
   d.maxuv = d.minuv + ctx->numslv + 1;
   CK(palloc(ctx, &d.edens_part, (size_t)kEdensSlices * ctx->ermax));
   if (p.corrcal) CK(palloc(ctx, &d.ecorr, (size_t)ctx->ermax * ctx->ermax));
-  CK(palloc(ctx, &d.status, 1)); CK(palloc(ctx, &d.frame_i, 4));
-  {   // pinned: the staged scalars, the status word, the accumulators' image and a frame's inputs
-    const size_t acc = sizeof(double) * acc_words(ctx), in = sizeof(float) * (3 * NA + MD);
-    CK(cudaMallocHost((void**)&ctx->h_block, 128 + acc + in));
-    ctx->h_frame = (int*)ctx->h_block;
-    ctx->h_status = (DevStatus*)(ctx->h_block + 64);
-    ctx->h_acc = (double*)(ctx->h_block + 128);
-    ctx->h_pin = (float*)(ctx->h_block + 128 + acc);
+  CK(palloc(ctx, (unsigned char**)&d.status, frame_zero_bytes(ctx)));
+  d.etot = (double*)((unsigned char*)d.status + 64);
+  d.selfrec = d.etot + MD;
+  d.flceng = d.selfrec + MD;
+  {   // pinned: the status word (with etot, selfrec and flceng behind it for solutions), the
+      // accumulators' image and a frame's inputs
+    const size_t acc = sizeof(double) * acc_words(ctx), in = in_bytes(ctx, 0);
+    const size_t status = (64 + (refs ? 0 : frame_zero_bytes(ctx)) + 63) / 64 * 64;
+    CK(cudaMallocHost((void**)&ctx->h_block, status + acc + in));
+    ctx->h_status = (DevStatus*)ctx->h_block;
+    ctx->h_acc = (double*)(ctx->h_block + status);
+    ctx->h_pin = ctx->h_block + status + acc;
     ctx->h_pin_bytes = in;
   }
   if (p.graph_mode < 0 || p.graph_mode > 1 || p.stage_timing < 0 || p.stage_timing > 1) return bad(ERMOD_ERR_ARG, "opt_arg");
@@ -1004,9 +1022,19 @@ static int frame_enqueue(ermod_ctx* ctx, const FramePlan& fp, cudaStream_t st, b
   const bool refs = p.slttype != ERMOD_SLT_SOLN;
   const bool pme = a.pme;
   auto M = [&](int tag) { if (timed) mark(ctx, tag); };
-  CK(cudaMemsetAsync(d.status, 0, sizeof(DevStatus), st));
-  launch_prepare_solvent(a, d, st);
-  launch_cells(a, d, fp.ncell, st);
+  // status word, etot, selfrec and flceng share an allocation
+  CK(cudaMemsetAsync(d.status, 0, frame_zero_bytes(ctx), st));
+  // The solvent's preparation feeds real space and the gather only: with PME it runs on the second
+  // stream beside the insertion, the site tables and the first chunk's planes and lines.
+  const bool fork = pme && !timed;
+  cudaStream_t sp = fork ? ctx->st2 : st;
+  if (fork) {
+    CK(cudaEventRecord(ctx->ev_fork, st));
+    CK(cudaStreamWaitEvent(sp, ctx->ev_fork, 0));
+  }
+  launch_prepare_solvent(a, d, sp);
+  launch_cells(a, d, fp.ncell, sp);
+  if (fork) CK(cudaEventRecord(ctx->ev_prep, sp));
   nl += 1 + (a.slvmax > 0 ? (a.use_cells ? 4 : 3) : 0);
   M(kStPrep);
   // ---- targets ----
@@ -1044,9 +1072,6 @@ static int frame_enqueue(ermod_ctx* ctx, const FramePlan& fp, cudaStream_t st, b
     launch_soln_region(a, d, ck, st);
     nl += 1;
   }
-  CK(cudaMemsetAsync(d.selfrec, 0, sizeof(double) * ctx->maxdst, st));
-  CK(cudaMemsetAsync(d.etot, 0, sizeof(double) * ctx->maxdst, st));
-  CK(cudaMemsetAsync(d.flceng, 0, sizeof(double) * ctx->maxdst * ctx->numslv, st));
   if (d.uvengy) CK(cudaMemsetAsync(d.uvengy, 0, sizeof(double) * ctx->maxdst * ctx->slvmax, st));
   switch (fp.selfreal) {
     case 0: CK(cudaMemsetAsync(d.selfreal, 0, sizeof(double) * ctx->maxdst, st)); break;
@@ -1061,13 +1086,13 @@ static int frame_enqueue(ermod_ctx* ctx, const FramePlan& fp, cudaStream_t st, b
   for (int bb = 0; bb < ctx->maxdst; bb += ctx->batch) {
     const int nbatch = std::min(ctx->batch, ctx->maxdst - bb);
     if (ctx->real_threads == 0) {
+      if (fork) CK(cudaStreamWaitEvent(st, ctx->ev_prep, 0));
       const int rc = tune_real(ctx, a, nbatch, st);
       if (rc != ERMOD_OK) return rc;
     }
     // Real space beside the PME chain: k_real on the second stream, joined before binning (the
     // gather writes the reciprocal part, k_bin adds the real part).  Stage-timed runs keep one
     // stream so that each stage's events bracket it alone; the arithmetic is the same.
-    const bool fork = pme && !timed;
     if (fork) {
       CK(cudaEventRecord(ctx->ev_fork, st));
       CK(cudaStreamWaitEvent(ctx->st2, ctx->ev_fork, 0));
@@ -1107,7 +1132,10 @@ static int frame_enqueue(ermod_ctx* ctx, const FramePlan& fp, cudaStream_t st, b
         M(kStTranspose);
         nl += 1;
       }
-      launch_gather(a, d, cb, bb, nb, chunk, ctx->batch, pdl, st);
+      // the frame's first gather waits for the solvent's preparation (a whole dependency, so launched
+      // without the programmatic one; the later gathers come behind it)
+      if (fork && cb == 0) CK(cudaStreamWaitEvent(st, ctx->ev_prep, 0));
+      launch_gather(a, d, cb, bb, nb, chunk, ctx->batch, pdl && cb > 0, st);
       M(kStGather);
       nl += 1;
     }
@@ -1120,7 +1148,7 @@ static int frame_enqueue(ermod_ctx* ctx, const FramePlan& fp, cudaStream_t st, b
                          cudaMemcpyDeviceToDevice, st));
     launch_weights(d, fp.wa, bb, nbatch, st);
     launch_edens(d, bb, nbatch, ctx->ermax, ctx->ermax_pad, bb, st);
-    nl += 3;
+    nl += 1 + (nbatch <= kEdensSlices ? 1 : 2);
     M(kStWeights);
     if (p.corrcal) {
       if (ctx->use_tc) {
@@ -1135,7 +1163,9 @@ static int frame_enqueue(ermod_ctx* ctx, const FramePlan& fp, cudaStream_t st, b
     }
     M(kStEcorr);
   }
-  CK(cudaMemcpyAsync(ctx->h_status, d.status, sizeof(DevStatus), cudaMemcpyDeviceToHost, st));
+  // the status word, for solutions with flceng behind it
+  CK(cudaMemcpyAsync(ctx->h_status, d.status, refs ? sizeof(DevStatus) : frame_zero_bytes(ctx), cudaMemcpyDeviceToHost,
+                     st));
   return ERMOD_OK;
 }
 
@@ -1195,13 +1225,15 @@ static cudaError_t capture_graph(cudaStream_t st, cudaGraphExec_t* exec, Body bo
 }
 
 // One frame of one context, its inputs already staged on ctx->st.
-static int engconst_run(ermod_ctx* ctx, int stnum, const float* cellin, float wsys, bool use_conf) {
+static int engconst_run(ermod_ctx* ctx, int stnum, bool staged, const float* cellin, float wsys, bool use_conf) {
   FramePlanHost ph;
   int rc = frame_plan(ctx, cellin, wsys, use_conf, ph);
   if (rc != ERMOD_OK) return rc;
   cudaStream_t st = ctx->st;
-  ctx->h_frame[0] = stnum;
-  CK(cudaMemcpyAsync(ctx->d.frame_i, ctx->h_frame, sizeof(int), cudaMemcpyHostToDevice, st));
+  if (!staged) {
+    *(int*)ctx->h_pin = stnum;
+    CK(cudaMemcpyAsync(ctx->d.frame_i, ctx->h_pin, sizeof(int), cudaMemcpyHostToDevice, st));
+  }
   if (ph.engfac) launch_engfac(ph.k.a, ctx->d, ph.inv, ph.vold, (double)ctx->p.screen, ctx->pppm, st);
   const bool timed = ctx->p.stage_timing != 0;
   const bool graph = !timed && ctx->p.graph_mode == 0 && ctx->real_threads != 0;
@@ -1239,16 +1271,16 @@ static int engconst_run(ermod_ctx* ctx, int stnum, const float* cellin, float ws
   return frame_finish(ctx, timed, total);
 }
 
-// Stage the host inputs of a frame into the context's device buffers.
-static int stage_host_inputs(ermod_ctx* ctx, const float* sitepos, const float* ins_conf, const float* ins_weight,
-                             size_t* nconf_out) {
+// Stage the host inputs of a frame into the context's device buffers, in one copy.
+static int stage_host_inputs(ermod_ctx* ctx, int stnum, const float* sitepos, const float* ins_conf,
+                             const float* ins_weight, size_t* nconf_out) {
   const bool refs = ctx->p.slttype != ERMOD_SLT_SOLN;
   const size_t npos = 3 * (size_t)ctx->natoms;
   const size_t nconf = (refs && ins_conf) ? 3 * (size_t)ctx->s * ctx->maxdst : 0;
-  const size_t need = sizeof(float) * (npos + nconf + ctx->maxdst);
+  const size_t need = in_bytes(ctx, nconf);
   if (ctx->h_pin_bytes < need) {
     // the new buffer first: should it fail, the context keeps the old one
-    float* grown = nullptr;
+    unsigned char* grown = nullptr;
     CK(cudaMallocHost((void**)&grown, need));
     CK(cudaStreamSynchronize(ctx->st));   // the old one may still feed the previous frame's copies
     if (ctx->h_grown) cudaFreeHost(ctx->h_grown);
@@ -1256,15 +1288,13 @@ static int stage_host_inputs(ermod_ctx* ctx, const float* sitepos, const float* 
     ctx->h_pin_bytes = need;
   }
   CK(cudaStreamSynchronize(ctx->st));   // the staging buffer may still feed the previous frame's copies
-  std::memcpy(ctx->h_pin, sitepos, sizeof(float) * npos);
-  CK(cudaMemcpyAsync(ctx->d.posraw, ctx->h_pin, sizeof(float) * npos, cudaMemcpyHostToDevice, ctx->st));
-  if (nconf) {
-    std::memcpy(ctx->h_pin + npos, ins_conf, sizeof(float) * nconf);
-    CK(cudaMemcpyAsync(ctx->d.ins_conf, ctx->h_pin + npos, sizeof(float) * nconf, cudaMemcpyHostToDevice, ctx->st));
-  }
-  float* hw = ctx->h_pin + npos + nconf;
+  *(int*)ctx->h_pin = stnum;
+  float* hw = (float*)(ctx->h_pin + kInHead);
   for (int i = 0; i < ctx->maxdst; ++i) hw[i] = (refs && ins_weight) ? ins_weight[i] : 1.0f;
-  CK(cudaMemcpyAsync(ctx->d.insw_in, hw, sizeof(float) * ctx->maxdst, cudaMemcpyHostToDevice, ctx->st));
+  float* pos = hw + ctx->maxdst;
+  std::memcpy(pos, sitepos, sizeof(float) * npos);
+  if (nconf) std::memcpy(pos + npos, ins_conf, sizeof(float) * nconf);
+  CK(cudaMemcpyAsync(ctx->d.frame_i, ctx->h_pin, need, cudaMemcpyHostToDevice, ctx->st));
   *nconf_out = nconf;
   return ERMOD_OK;
 }
@@ -1278,14 +1308,13 @@ int32_t ermod_engconst(ermod_ctx* ctx, int32_t stnum, const float* sitepos, cons
   CK(cudaSetDevice(ctx->device));
   const bool refs = ctx->p.slttype != ERMOD_SLT_SOLN;
   size_t nconf = 0;
-  int rc = stage_host_inputs(ctx, sitepos, ins_conf, ins_weight, &nconf);
+  int rc = stage_host_inputs(ctx, stnum, sitepos, ins_conf, ins_weight, &nconf);
   if (rc != ERMOD_OK) return rc;
-  rc = engconst_run(ctx, stnum, cell, stat_weight_system, nconf > 0);
+  rc = engconst_run(ctx, stnum, true, cell, stat_weight_system, nconf > 0);
   if (rc < 0) return rc;
   if (flceng && !refs) {
-    std::vector<double> f((size_t)ctx->maxdst * ctx->numslv);
-    CK(cudaMemcpy(f.data(), ctx->d.flceng, sizeof(double) * f.size(), cudaMemcpyDeviceToHost));
-    for (size_t i = 0; i < f.size(); ++i) flceng[i] = (float)f[i];
+    const double* f = (const double*)((const char*)ctx->h_status + ((const char*)ctx->d.flceng - (const char*)ctx->d.status));
+    for (size_t i = 0; i < (size_t)ctx->maxdst * ctx->numslv; ++i) flceng[i] = (float)f[i];
   }
   return rc;
 }
@@ -1304,7 +1333,7 @@ int32_t ermod_engconst_dev(ermod_ctx* ctx, int32_t stnum, const float* sitepos_d
     CK(cudaMemcpyAsync(ctx->d.insw_in, ins_weight_dev, sizeof(float) * ctx->maxdst, cudaMemcpyDeviceToDevice, ctx->st));
   else
     launch_fill(ctx->d.insw_in, 1.0f, ctx->maxdst, ctx->st);
-  return engconst_run(ctx, stnum, cell, stat_weight_system, refs && ins_conf_dev);
+  return engconst_run(ctx, stnum, false, cell, stat_weight_system, refs && ins_conf_dev);
 }
 
 // ---- batches of contexts: one graph launch per frame ---------------------
@@ -1397,8 +1426,8 @@ static int batch_run(ermod_batch* b, int stnum, const float* cell, float wsys) {
     if (cudaMemcpyAsync(ctx->d.posraw, b->d_pos, sizeof(float) * b->npos, cudaMemcpyDeviceToDevice, b->st) !=
         cudaSuccess)
       return ERMOD_ERR_CUDA;
-    ctx->h_frame[0] = stnum;
-    if (cudaMemcpyAsync(ctx->d.frame_i, ctx->h_frame, sizeof(int), cudaMemcpyHostToDevice, b->st) != cudaSuccess)
+    *(int*)ctx->h_pin = stnum;
+    if (cudaMemcpyAsync(ctx->d.frame_i, ctx->h_pin, sizeof(int), cudaMemcpyHostToDevice, b->st) != cudaSuccess)
       return ERMOD_ERR_CUDA;
     launch_fill(ctx->d.insw_in, 1.0f, ctx->maxdst, b->st);
     if (ph[i].engfac) launch_engfac(ph[i].k.a, ctx->d, ph[i].inv, ph[i].vold, (double)ctx->p.screen, ctx->pppm, b->st);

@@ -54,11 +54,13 @@ __global__ void k_prepare_solvent(FrameArgs a, const float* __restrict__ posraw,
       const float f = inm[m] * (float)K[m];
       const int rci = (int)f;
       spline_weights(f - (float)rci, a.order, wr[m]);
-      for (int spi = 0; spi < a.order; ++spi) spl[((size_t)i * 3 + m) * a.order + spi] = wr[m][spi];
       gi[m] = rci;
     }
-    grd[i] = make_int4(gi[0], gi[1], gi[2], 0);
-    if (grec) {   // order 4 (gather_rec_ok)
+    if (!grec) {  // k_gather's tables
+      for (int m = 0; m < 3; ++m)
+        for (int spi = 0; spi < a.order; ++spi) spl[((size_t)i * 3 + m) * a.order + spi] = wr[m][spi];
+      grd[i] = make_int4(gi[0], gi[1], gi[2], 0);
+    } else {      // order 4 (gather_rec_ok): k_gather_rec's and k_gather_few's records
       const float q = atom_q[i];
       const bool wrapx = !(gi[0] >= 3 && gi[0] < a.K1);
       const bool wrap = wrapx || !(gi[1] >= 3 && gi[2] >= 3 && gi[1] < a.K2 && gi[2] < a.K3);
@@ -121,14 +123,15 @@ __global__ void k_anchor(FrameArgs a, const int* __restrict__ molbeg, const floa
   if (k >= a.slvmax) return;
   const int b0 = molbeg[k], b1 = molbeg[k + 1];
   const float4 p0 = slvn[b0];
-  float ext = 0.0f;
+  float ext2 = 0.0f;
+#pragma unroll 4
   for (int at = b0 + 1; at < b1; ++at) {
     const float4 q = slvn[at];
     float dx = q.x - p0.x, dy = q.y - p0.y, dz = q.z - p0.z;
     min_image(a.g, dx, dy, dz);
-    ext = fmaxf(ext, sqrtf(dx * dx + dy * dy + dz * dz));
+    ext2 = fmaxf(ext2, dx * dx + dy * dy + dz * dz);
   }
-  anchor[k] = make_float4(p0.x, p0.y, p0.z, ext);
+  anchor[k] = make_float4(p0.x, p0.y, p0.z, sqrtf(ext2));
   if (a.use_cells) {
     const int cx = cell_coord(p0.x, a.ch[0], a.nc[0]);
     const int cy = cell_coord(p0.y, a.ch[1], a.nc[1]);
@@ -1887,41 +1890,51 @@ cudaError_t raise_smem_limit_fn(const void* kernel, size_t bytes) {
 // ---------------------------------------------------------------------------
 // weights and accumulators
 // ---------------------------------------------------------------------------
-__global__ void k_offset_init(WeightArgs wa, int base, int n, const int* __restrict__ skip,
-                              const double* __restrict__ selfrec, const double* __restrict__ selfreal,
-                              double* __restrict__ scal) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  int c = base;   // the first target not rejected (engproc.F90:447-450)
-  if (skip) while (c < base + n && skip[c]) ++c;
-  if (c >= base + n) return;
-  if (wa.rigid && scal[6] == 0.0) { scal[5] = selfreal[c]; scal[6] = 1.0; }
-  if (wa.wgtslf && scal[4] == 0.0) {
-    const double sr = wa.rigid ? scal[5] : selfreal[c];
-    scal[3] = selfrec[c] + sr + wa.resid_self;
-    scal[4] = 1.0;
-  }
-}
+// One CTA for a batch: the offset, every target's weight engnmfc (engproc.F90:883-903, volcorrect
+// :1022-1038) and the batch's scalar accumulators, summed in a fixed order (engproc.F90:905-915,
+// 939-941): engnorm, engsmpl, avslf, the self-energy histogram, slnuv (soln) and the self-energy
+// min / max.  At most 4096 targets, four a thread.  One target: 3.5 us, where a launch each for offset,
+// weights and sums took 8 with their gaps.
+constexpr int kSumThreads = 1024;
 
-// per-target weight engnmfc (engproc.F90:883-903, volcorrect :1022-1038)
-__global__ void k_weights(WeightArgs wa, int base, int n, const int* __restrict__ skip,
-                          const double* __restrict__ selfrec, const double* __restrict__ selfreal,
-                          const float* __restrict__ insw,
-                          const double* __restrict__ escrd, double* __restrict__ u0, double* __restrict__ w,
-                          double* __restrict__ twt, int* __restrict__ sbin, const double* __restrict__ scal,
-                          DevStatus* st) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) {
+__global__ void __launch_bounds__(kSumThreads) k_weights(WeightArgs wa, int base, int n, const int* __restrict__ skip,
+    const double* __restrict__ selfrec, const double* __restrict__ selfreal, const float* __restrict__ insw,
+    const double* __restrict__ escrd, double* __restrict__ u0, double* __restrict__ w, double* __restrict__ twt,
+    int* __restrict__ sbin, const double* __restrict__ flceng, double* __restrict__ scal, double* __restrict__ eself,
+    double* __restrict__ slnuv, float* __restrict__ minuv, float* __restrict__ maxuv, DevStatus* st) {
+  __shared__ double r0[32], r1[32], ref[2];
+  __shared__ float rm[32], rx[32];
+  __shared__ int rk[32];
+  if (threadIdx.x == 0) {
+    int c = base;   // the first target not rejected (engproc.F90:447-450)
+    if (skip) while (c < base + n && skip[c]) ++c;
+    if (c < base + n) {
+      if (wa.rigid && scal[6] == 0.0) { scal[5] = selfreal[c]; scal[6] = 1.0; }
+      if (wa.wgtslf && scal[4] == 0.0) {
+        const double sr = wa.rigid ? scal[5] : selfreal[c];
+        scal[3] = selfrec[c] + sr + wa.resid_self;
+        scal[4] = 1.0;
+      }
+    }
+    ref[0] = scal[3];
+    ref[1] = scal[5];
+  }
+  __syncthreads();
+  const double voffset = ref[0], usreal = ref[1];
+  double a0 = 0.0, a1 = 0.0;
+  float mn = FLT_MAX, mx = -FLT_MAX;
+  int kept = 0;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const int cnt = base + i;
-    double tw;
-    const double sr = wa.rigid ? scal[5] : selfreal[cnt];
+    const double sr = wa.rigid ? usreal : selfreal[cnt];
     const double uu = selfrec[cnt] + sr + wa.resid_self;
     u0[cnt] = uu;
     double e = 1.0;
     if (wa.wgtslf) {
-      const double f = uu - scal[3];
+      const double f = uu - voffset;
       e = wa.slttype == ERMOD_SLT_SOLN ? exp(f / wa.temp) : exp(-f / wa.temp);
     }
-    tw = (double)wa.stat_weight_system * (double)insw[cnt] * wa.npt_factor;
+    const double tw = (double)wa.stat_weight_system * (double)insw[cnt] * wa.npt_factor;
     e *= tw;
     const bool rej = skip && skip[cnt];   // rejected: no update_histogram (engproc.F90:447-450)
     w[cnt] = rej ? 0.0 : e;
@@ -1939,30 +1952,10 @@ __global__ void k_weights(WeightArgs wa, int base, int n, const int* __restrict_
       }
     }
     sbin[cnt] = l;
-  }
-}
-
-// Scalar accumulators of one batch, summed in a fixed order by one CTA
-// (engproc.F90:905-915, 939-941): engnorm, engsmpl, avslf, the self-energy
-// histogram, slnuv (soln) and the self-energy min / max.
-constexpr int kSumThreads = 1024;
-
-__global__ void __launch_bounds__(kSumThreads) k_wsum(WeightArgs wa, int base, int n, const int* __restrict__ skip,
-    const double* __restrict__ w, const double* __restrict__ twt, const double* __restrict__ u0,
-    const int* __restrict__ sbin,
-    const double* __restrict__ flceng, double* __restrict__ scal, double* __restrict__ eself,
-    double* __restrict__ slnuv, float* __restrict__ minuv, float* __restrict__ maxuv) {
-  __shared__ double r0[32], r1[32];
-  __shared__ float rm[32], rx[32];
-  __shared__ int rk[32];
-  double a0 = 0.0, a1 = 0.0;
-  float mn = FLT_MAX, mx = -FLT_MAX;
-  int kept = 0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    if (skip && skip[base + i]) continue;
-    a0 += w[base + i];
-    a1 += twt[base + i];
-    const float u = (float)u0[base + i];
+    if (rej) continue;
+    a0 += e;
+    a1 += tw;
+    const float u = (float)uu;
     mn = fminf(mn, u);
     mx = fmaxf(mx, u);
     ++kept;
@@ -1973,7 +1966,7 @@ __global__ void __launch_bounds__(kSumThreads) k_wsum(WeightArgs wa, int base, i
     r0[threadIdx.x >> 5] = a0; r1[threadIdx.x >> 5] = a1; rm[threadIdx.x >> 5] = mn; rx[threadIdx.x >> 5] = mx;
     rk[threadIdx.x >> 5] = kept;
   }
-  __syncthreads();
+  __syncthreads();   // also: every w and sbin is written
   if (threadIdx.x < 32) {
     const bool ok = threadIdx.x < (blockDim.x >> 5);
     a0 = warp_sum(ok ? r0[threadIdx.x] : 0.0);
@@ -2007,11 +2000,8 @@ __global__ void __launch_bounds__(kSumThreads) k_wsum(WeightArgs wa, int base, i
 
 void launch_weights(const DeviceState& d, const WeightArgs& wa, int base, int n, cudaStream_t s) {
   if (n <= 0) return;
-  k_offset_init<<<1, 32, 0, s>>>(wa, base, n, d.skip, d.selfrec, d.selfreal, d.scal);
-  k_weights<<<(n + 255) / 256, 256, 0, s>>>(wa, base, n, d.skip, d.selfrec, d.selfreal, d.insw_in, d.escrd, d.u0,
-                                             d.w, d.twt, d.sbin, d.scal, d.status);
-  k_wsum<<<1, kSumThreads, 0, s>>>(wa, base, n, d.skip, d.w, d.twt, d.u0, d.sbin, d.flceng, d.scal, d.eself,
-                                   d.slnuv, d.minuv, d.maxuv);
+  k_weights<<<1, std::min(kSumThreads, (n + 31) / 32 * 32), 0, s>>>(wa, base, n, d.skip, d.selfrec, d.selfreal,
+      d.insw_in, d.escrd, d.u0, d.w, d.twt, d.sbin, d.flceng, d.scal, d.eself, d.slnuv, d.minuv, d.maxuv, d.status);
 }
 
 __global__ void k_edens(int base, int n, int ermax, int ermax_pad, int count_base, const double* __restrict__ w,
@@ -2052,7 +2042,7 @@ __global__ void k_edens_sum(int ermax, int ns, const double* __restrict__ part, 
 
 void launch_edens(const DeviceState& d, int base, int n, int ermax, int ermax_pad, int count_base, cudaStream_t s) {
   if (n <= 0) return;
-  if (!d.edens_part) {
+  if (!d.edens_part || n <= kEdensSlices) {   // a slice would hold at most one target: the same sums, one launch
     k_edens<<<(ermax + 127) / 128, 128, 0, s>>>(base, n, ermax, ermax_pad, count_base, d.w, d.counts, d.edens);
     return;
   }
