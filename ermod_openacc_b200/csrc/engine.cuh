@@ -95,6 +95,15 @@ __host__ __device__ __forceinline__ bool gather_rec_ok(int order, int K1, int K2
          (double)K3 * K2 * (((K1 + 1) / 2) * 2) * 32 < 2147483647.0;
 }
 
+// Chunks of at most this many targets (solution frames have one) on the fused solve's meshes up to
+// K1 = 64 keep their potential grids in natural order, [target][n3][n2][n1], with kernels whose lanes
+// are lines and molecules' stencil planes (k_pme_lines_few, k_gather_few); larger ones one lane a
+// target.  Line and gather stage of 4096 waters on a 64^3 mesh, lanes over targets against these:
+// 36 / 19 us at one target, 36 / 23 at four, 35 / 29 at eight, 36 / 50 at sixteen.
+constexpr int kFewTargets = 8;
+struct DeviceState;
+bool few_targets(const FrameArgs& a, const DeviceState& d, int nb);
+
 // Float offset of phi(n1) of grid line `line` (= n3 K2 + n2) and target b in the
 // pair layout: n1 pairs of kChunk targets, P1 = ceil(K1 / 2) pairs per line.
 __host__ __device__ __forceinline__ size_t phi_index(size_t line, int n1, int b, int P1) {

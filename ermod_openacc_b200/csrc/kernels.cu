@@ -1697,9 +1697,64 @@ __global__ void __launch_bounds__(kGatherThreads, 4) k_gather_rec(FrameArgs a, i
   }
 }
 
+bool few_targets(const FrameArgs& a, const DeviceState& d, int nb) {
+  return nb <= kFewTargets && a.pme && a.order == 4 && d.grec && d.engfacT && a.K1 <= 64;
+}
+
+// The order-4 gather for few targets, potential grids in natural order: four lanes a (molecule,
+// target), lane = stencil plane c3, the 16 points of a plane in flight together; a plane's FP32 sum
+// and its FP64 share are k_gather_rec's, the four shares and the atoms are added in a fixed order.
+// One target, 4096 waters, 64^3 mesh: 41 us with lanes over targets and
+// the 60-site target's own atoms walked, 5.5 so.
+__global__ void __launch_bounds__(128) k_gather_few(FrameArgs a, int base, int bb, const int4* __restrict__ mrec,
+    const float* __restrict__ grec, const float* __restrict__ phi, const double* __restrict__ tgtq,
+    const int* __restrict__ tgt_mol, double* __restrict__ Etot) {
+  const int m = (blockIdx.x * blockDim.x + threadIdx.x) >> 2, c3 = threadIdx.x & 3, b = blockIdx.y;
+  const int cnt = base + b, bi = cnt - bb, K1 = a.K1, K2 = a.K2, K3 = a.K3;
+  grid_dep_wait();                                    // the potential grid of this chunk is complete
+  grid_dep_launch();
+  const bool on = m < a.slvmax;
+  int4 mr = on ? mrec[m] : make_int4(0, 0, 0, 0);
+  const bool excl = on && tgt_mol && mr.x == tgt_mol[cnt];   // the target itself, often the largest molecule
+  if (excl) mr.z = 0;
+  const float* grid = phi + (size_t)b * K3 * K2 * K1;
+  double e = 0.0;
+  for (int at = 0; at < mr.z; ++at) {
+    const float4* r4 = (const float4*)(grec + (size_t)(mr.y + at) * kRecWords);
+    const float4 w1 = r4[0], w2 = r4[1], w3 = r4[2];
+    const int gp = __float_as_int(r4[3].z);
+    const int gx = gp & 1023, gy = (gp >> 10) & 1023, gz = gp >> 20;
+    const float w[9] = {w1.x, w1.y, w1.z, w1.w, w2.x, w2.y, w2.z, w2.w,
+                        c3 == 0 ? w3.x : c3 == 1 ? w3.y : c3 == 2 ? w3.z : w3.w};
+    const float* pl = grid + (size_t)wrapk(gz - c3, K3) * K2 * K1;
+    int n1[4];
+    float v[16];
+#pragma unroll
+    for (int c1 = 0; c1 < 4; ++c1) n1[c1] = wrapk(gx - c1, K1);
+#pragma unroll
+    for (int c2 = 0; c2 < 4; ++c2) {
+      const float* row = pl + wrapk(gy - c2, K2) * K1;
+#pragma unroll
+      for (int c1 = 0; c1 < 4; ++c1) v[c2 * 4 + c1] = row[n1[c1]];
+    }
+    accumulate_planes<4, 1>(v, w, 0, 1.0f, e);        // w[8] is q w3(c3)
+  }
+  e += __shfl_xor_sync(0xffffffffu, e, 1);
+  e += __shfl_xor_sync(0xffffffffu, e, 2);
+  if (on && c3 == 0) {
+    e -= a.pivol * tgtq[cnt] * (double)__int_as_float(mr.w);
+    Etot[(size_t)bi * a.slvmax + mr.x] = excl ? 0.0 : e;
+  }
+}
+
 void launch_gather(const FrameArgs& a, const DeviceState& d, int base, int bb, int nb, int chunk, int batch,
                    bool pdl, cudaStream_t s) {
   int blocks = (a.slvmax * 32 + kGatherThreads - 1) / kGatherThreads;
+  if (few_targets(a, d, nb)) {
+    launch_k(pdl, dim3((a.slvmax * 4 + 127) / 128, nb), 128, 0, s, k_gather_few, a, base, bb, (const int4*)d.mrec,
+             (const float*)d.grec, (const float*)d.phi, (const double*)d.tgtq, (const int*)d.tgt_mol, d.Etot);
+    return;
+  }
   if (a.pme && a.order == 4 && d.grec) {
     // no more CTAs than are resident at once: every warp fetches its first records early
     static std::atomic<int> resident[kMaxDevices];
