@@ -311,88 +311,73 @@ __device__ uint32_t site_mma(const float2* __restrict__ tab, size_t pairA, int k
         }
       }
     }
-    if constexpr (KN == 128) {
-      // 128 x 128 planes (one target, one plane): consecutive lanes take consecutive k2 and k3,
-      // so the table reads are 256-byte runs.  Measured on the 60-site chain, this order keeps
-      // the plane stage at 43 ms a frame where the bank-conflict-free order below took 48.
-      for (int e = tid; e < ns * KN; e += NTHR) {
-        const int t = e / KN, q = e - t * KN;
-        const float2* row = tab + (pairA + t0 + t) * nk;
-        const float2 d = fft::cmul(row[k1A], row[Kh1 + q]);   // q B1(k1) B2(k2 = q)
-        put_split2(ahi, alo, q, 2 * t, d.x, d.y);
-        const float2 b3 = row[Kh1 + KN + q];                  // B3(k3 = q)
-        put_split2(bhi, blo, 2 * q, 2 * t, b3.x, -b3.y);
-        put_split2(bhi, blo, 2 * q + 1, 2 * t, b3.y, b3.x);
-      }
-    } else {
-      // The item orders put the 16 lanes of a half warp on 16 distinct (16-byte chunk, half)
-      // slots of the swizzled rows, so the 8-byte stores are free of bank conflicts: a lane's
-      // chunk is (t / 2) ^ (row mod 8), its half t mod 2.
-      // A rows k2 = q: item bits 0-2 q mod 8, bit 3 t mod 2, bits 4.. q / 8, then t / 2.  Each
-      // loop loads NB items of the thread at a time, then splits and stores them, so that the
-      // table reads are in flight together.
+    // The item orders put the 16 lanes of a half warp on 16 distinct (16-byte chunk, half)
+    // slots of the swizzled rows, so the 8-byte stores are free of bank conflicts: a lane's
+    // chunk is (t / 2) ^ (row mod 8), its half t mod 2.
+    // A rows k2 = q: item bits 0-2 q mod 8, bit 3 t mod 2, bits 4.. q / 8, then t / 2.  Each
+    // loop loads NB items of the thread at a time, then splits and stores them, so that the
+    // table reads are in flight together.
 #pragma unroll 1
-      for (int u0 = 0; u0 < NI; u0 += NB) {
-        const int lim = ((ns + 1) >> 1) * 2 * KN;
-        const bool same = pairB == pairA;
-        float2 c1v[NB], b2v[NB], c1w[NB], b2w[NB];
+    for (int u0 = 0; u0 < NI; u0 += NB) {
+      const int lim = ((ns + 1) >> 1) * 2 * KN;
+      const bool same = pairB == pairA;
+      float2 c1v[NB], b2v[NB], c1w[NB], b2w[NB];
 #pragma unroll
-        for (int u = 0; u < NB; ++u) {
-          const int x = tid + (u0 + u) * NTHR;
-          const int q = (x & 7) | (((x >> 4) & (KN / 8 - 1)) << 3);
-          const int t = ((x >> 3) & 1) | ((x / (2 * KN)) << 1);
-          const float2 z = make_float2(0.f, 0.f);
-          c1v[u] = z; b2v[u] = z; c1w[u] = z; b2w[u] = z;
-          if (x < lim && t < ns) {
-            const float2* row = tab + (pairA + t0 + t) * nk;
-            b2v[u] = row[Kh1 + q];
-            if (onA) c1v[u] = row[k1A];
-            if (KN == 64 && onB) {
-              const float2* rb = same ? row : tab + (pairB + t0 + t) * nk;
-              c1w[u] = rb[k1B];
-              if (!same) b2w[u] = rb[Kh1 + q];
-            }
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < NB; ++u) {
-          const int x = tid + (u0 + u) * NTHR;
-          const int q = (x & 7) | (((x >> 4) & (KN / 8 - 1)) << 3);
-          const int t = ((x >> 3) & 1) | ((x / (2 * KN)) << 1);
-          if (x < lim && t < ns) {
-            const float2 d = fft::cmul(c1v[u], b2v[u]);       // q B1(k1) B2(k2 = q); zero when off
-            put_split2(ahi, alo, q, 2 * t, d.x, d.y);
-            if (KN == 64) {
-              const float2 e = fft::cmul(c1w[u], same ? b2v[u] : b2w[u]);
-              put_split2(ahi, alo, 64 + q, 2 * t, e.x, e.y);
-            }
+      for (int u = 0; u < NB; ++u) {
+        const int x = tid + (u0 + u) * NTHR;
+        const int q = (x & 7) | (((x >> 4) & (KN / 8 - 1)) << 3);
+        const int t = ((x >> 3) & 1) | ((x / (2 * KN)) << 1);
+        const float2 z = make_float2(0.f, 0.f);
+        c1v[u] = z; b2v[u] = z; c1w[u] = z; b2w[u] = z;
+        if (x < lim && t < ns) {
+          const float2* row = tab + (pairA + t0 + t) * nk;
+          b2v[u] = row[Kh1 + q];
+          if (onA) c1v[u] = row[k1A];
+          if (KN == 64 && onB) {
+            const float2* rb = same ? row : tab + (pairB + t0 + t) * nk;
+            c1w[u] = rb[k1B];
+            if (!same) b2w[u] = rb[Kh1 + q];
           }
         }
       }
-      // B row pairs (2 c2, 2 c2 + 1): item bits 0-1 c2 mod 4, bits 2-3 t mod 4, bits 4.. c2 / 4,
-      // then t / 4.  Pair c2 holds k3 = c2.
-#pragma unroll 1
-      for (int u0 = 0; u0 < NI; u0 += NB) {
-        const int lim = ((ns + 3) >> 2) * 4 * KN;
-        float2 v[NB];
 #pragma unroll
-        for (int u = 0; u < NB; ++u) {
-          const int x = tid + (u0 + u) * NTHR;
-          const int c2 = (x & 3) | (((x >> 4) & (KN / 4 - 1)) << 2);
-          const int t = ((x >> 2) & 3) | ((x / (4 * KN)) << 2);
-          const int k3 = c2;
-          v[u] = make_float2(0.f, 0.f);
-          if (x < lim && t < ns) v[u] = tab[(pb3 + t0 + t) * nk + Kh1 + KN + k3];
-        }
-#pragma unroll
-        for (int u = 0; u < NB; ++u) {
-          const int x = tid + (u0 + u) * NTHR;
-          const int c2 = (x & 3) | (((x >> 4) & (KN / 4 - 1)) << 2);
-          const int t = ((x >> 2) & 3) | ((x / (4 * KN)) << 2);
-          if (x < lim && t < ns) {
-            put_split2(bhi, blo, 2 * c2, 2 * t, v[u].x, -v[u].y);
-            put_split2(bhi, blo, 2 * c2 + 1, 2 * t, v[u].y, v[u].x);
+      for (int u = 0; u < NB; ++u) {
+        const int x = tid + (u0 + u) * NTHR;
+        const int q = (x & 7) | (((x >> 4) & (KN / 8 - 1)) << 3);
+        const int t = ((x >> 3) & 1) | ((x / (2 * KN)) << 1);
+        if (x < lim && t < ns) {
+          const float2 d = fft::cmul(c1v[u], b2v[u]);       // q B1(k1) B2(k2 = q); zero when off
+          put_split2(ahi, alo, q, 2 * t, d.x, d.y);
+          if (KN == 64) {
+            const float2 e = fft::cmul(c1w[u], same ? b2v[u] : b2w[u]);
+            put_split2(ahi, alo, 64 + q, 2 * t, e.x, e.y);
           }
+        }
+      }
+    }
+    // B row pairs (2 c2, 2 c2 + 1): item bits 0-1 c2 mod 4, bits 2-3 t mod 4, bits 4.. c2 / 4,
+    // then t / 4.  Pair c2 holds k3 = c2.
+#pragma unroll 1
+    for (int u0 = 0; u0 < NI; u0 += NB) {
+      const int lim = ((ns + 3) >> 2) * 4 * KN;
+      float2 v[NB];
+#pragma unroll
+      for (int u = 0; u < NB; ++u) {
+        const int x = tid + (u0 + u) * NTHR;
+        const int c2 = (x & 3) | (((x >> 4) & (KN / 4 - 1)) << 2);
+        const int t = ((x >> 2) & 3) | ((x / (4 * KN)) << 2);
+        const int k3 = c2;
+        v[u] = make_float2(0.f, 0.f);
+        if (x < lim && t < ns) v[u] = tab[(pb3 + t0 + t) * nk + Kh1 + KN + k3];
+      }
+#pragma unroll
+      for (int u = 0; u < NB; ++u) {
+        const int x = tid + (u0 + u) * NTHR;
+        const int c2 = (x & 3) | (((x >> 4) & (KN / 4 - 1)) << 2);
+        const int t = ((x >> 2) & 3) | ((x / (4 * KN)) << 2);
+        if (x < lim && t < ns) {
+          put_split2(bhi, blo, 2 * c2, 2 * t, v[u].x, -v[u].y);
+          put_split2(bhi, blo, 2 * c2 + 1, 2 * t, v[u].y, v[u].x);
         }
       }
     }
@@ -431,29 +416,100 @@ __device__ __forceinline__ void tmem_release(uint32_t tmem) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Shape<KN>::kTmemCols));
 }
 
-// X(k3, k2) of plane k1 of the target whose site tables start at pair0, straight into the
-// calling thread's registers in the plane kernel's layout: acc[e] = X(k30 + e, k2) with
-// k2 = tid mod KN, k30 = E (tid / KN).  The product is X^T: A(k2, 2 s + c) = (Re, Im) of
-// D_s(k2) = q B1_s(k1) B2_s(k2); B(2 k3 + p, 2 s + c) = (Re B3, -Im B3) for p = 0 and
-// (Im B3, Re B3) for p = 1.  Thread lane l of warp w reads TMEM lane 32 (w mod 4) + l, which
-// holds k2 = (32 w + l) mod KN, and the 2 E columns of its k3 range.  `opnd`
-// (Shape<KN>::kOperandBytes, 1024-byte aligned) may alias the plane buffer, which this
-// function does not write.  NTHR = KN * KN / E threads.
-template <int KN, int E, int NTHR>
-__device__ void site_sums(const float2* __restrict__ tab, size_t pair0, int s, int nk, int Kh1, int k1, int k30,
-                          unsigned char* opnd, uint64_t* bar, uint32_t* tmem_slot, int* __restrict__ errflags,
-                          float2 (&acc)[E]) {
-  static_assert(NTHR == KN * KN / E && (2 * E) % 32 == 0, "whole 32-column TMEM loads");
-  const uint32_t tmem = site_mma<KN, NTHR>(tab, pair0, k1, pair0, k1, s, nk, Kh1, opnd, bar, tmem_slot, errflags);
-  const int warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int c = 0; c < 2 * E; c += 32) {
-    uint32_t v[32];
-    tc::tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(2 * k30 + c), v);
-#pragma unroll
-    for (int j = 0; j < 16; ++j) acc[c / 2 + j] = make_float2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
+// The 128 x 128 plane's product: one target, one plane, tiles of 16 sites in two operand buffers
+// (Shape<128>::kOperandBytes each), so that a tile is staged while the tensor cores work on the one
+// before, from table values fetched a tile ahead.  The items are ordered as site_mma's, free of bank
+// conflicts (fetched a tile ahead, the shorter runs of table reads no longer cost what they save).
+// Bars: two mbarriers.  Returns the TMEM address of the product; 512 threads.
+__device__ __forceinline__ uint32_t site_mma128(const float2* __restrict__ tab, size_t pair0, int k1, int s, int nk,
+                                                int Kh1, unsigned char* opnd, uint64_t* bar, uint32_t* tmem_slot,
+                                                int* __restrict__ errflags) {
+  constexpr int KN = 128, NTHR = 512, NI = kTileSites * KN / NTHR;
+  using Sh = Shape<KN>;
+  using namespace tc;
+  const int tid = threadIdx.x;
+  // A item u: x = tid + 512 u, q = x bits 0-2 and 4-7, site x bits 3 and 8-10
+  // B item u: k3 = x bits 0-1 and 4-8, site x bits 2-3 and 9-10
+  const int qa = (tid & 7) | (((tid >> 4) & 15) << 3), ta = ((tid >> 3) & 1) | ((tid >> 8) << 1);
+  const int qb = (tid & 3) | (((tid >> 4) & 31) << 2), tb = (tid >> 2) & 3;
+  if (tid < 32) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"(Sh::kTmemCols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
-  tmem_release<KN>(tmem);
+  if (tid == 0) {
+    mbar_init(&bar[0], 1);
+    mbar_init(&bar[1], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  float2 c1[NI], b2[NI], b3[NI];
+  auto load = [&](int t0) {
+#pragma unroll
+    for (int u = 0; u < NI; ++u) {
+      const int t = t0 + ta + 4 * u, v = t0 + tb + 4 * u;
+      c1[u] = b2[u] = b3[u] = make_float2(0.f, 0.f);
+      if (t < s) {
+        const float2* row = tab + (pair0 + t) * nk;
+        c1[u] = __ldg(row + k1);
+        b2[u] = __ldg(row + Kh1 + qa);
+      }
+      if (v < s) b3[u] = __ldg(tab + (pair0 + v) * nk + Kh1 + KN + qb);
+    }
+  };
+  load(0);
+  bool ok = true;
+  uint32_t tmem = 0;
+  int tile = 0;
+  for (int t0 = 0; t0 < s && ok; t0 += kTileSites, ++tile) {
+    unsigned char* ahi = opnd + (tile & 1) * Sh::kOperandBytes;
+    unsigned char* alo = ahi + Sh::kAB;
+    unsigned char* bhi = alo + Sh::kAB;
+    unsigned char* blo = bhi + Sh::kBB;
+    if (tile >= 2) {   // the MMAs that read this buffer two tiles ago are done (bounded wait)
+      ok = __syncthreads_and(mbar_wait(&bar[tile & 1], (uint32_t)((tile >> 1) - 1) & 1u)) != 0;
+      if (!ok) break;
+    }
+    const int ns = min(kTileSites, s - t0), nks = (2 * ns + 7) / 8;
+#pragma unroll
+    for (int u = 0; u < NI; ++u) {   // sites past ns, up to the last K step's columns, are zeros
+      const int t = ta + 4 * u, v = tb + 4 * u;
+      if (t < 4 * nks) {
+        const float2 d = fft::cmul(c1[u], b2[u]);             // q B1(k1) B2(k2 = qa)
+        put_split2(ahi, alo, qa, 2 * t, d.x, d.y);
+      }
+      if (v < 4 * nks) {
+        put_split2(bhi, blo, 2 * qb, 2 * v, b3[u].x, -b3[u].y);       // B3(k3 = qb)
+        put_split2(bhi, blo, 2 * qb + 1, 2 * v, b3[u].y, b3[u].x);
+      }
+    }
+    load(t0 + kTileSites);
+    fence_proxy_async();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    tmem = *tmem_slot;
+    if (tid == 0) {
+      const uint64_t dah = smem_desc(smem_u32(ahi)), dal = smem_desc(smem_u32(alo));
+      const uint64_t dbh = smem_desc(smem_u32(bhi)), dbl = smem_desc(smem_u32(blo));
+      for (int ks = 0; ks < nks; ++ks)
+        mma(tmem, dah + 2 * ks, dbh + 2 * ks, Sh::kIdesc, (t0 > 0 || ks > 0) ? 1u : 0u);
+      for (int ks = 0; ks < nks; ++ks) mma(tmem, dah + 2 * ks, dbl + 2 * ks, Sh::kIdesc, 1u);
+      for (int ks = 0; ks < nks; ++ks) mma(tmem, dal + 2 * ks, dbh + 2 * ks, Sh::kIdesc, 1u);
+      mma_commit(&bar[tile & 1]);
+    }
+  }
+  // the last commit covers every MMA before it; on expiry of a wait the error is flagged and the kernel
+  // waits once more, bounded, before going on
+  const int last = tile - 1;
+  if (ok) ok = __syncthreads_and(mbar_wait(&bar[last & 1], (uint32_t)(last >> 1) & 1u)) != 0;
+  if (!ok) {
+    if (tid == 0) atomicOr(errflags, kErrTimeout);
+    const int w = tile > 0 ? tile - 1 : 0;
+    mbar_wait(&bar[w & 1], (uint32_t)(w >> 1) & 1u);
+    __syncthreads();
+  }
+  tc_fence_after();
+  return tmem;
 }
 }  // namespace tcs
 
@@ -462,11 +518,11 @@ __device__ void site_sums(const float2* __restrict__ tab, size_t pair0, int s, i
 // tid owns the points (k2 = tid mod K2, k3 = (tid / K2) * E + e), e < E.
 // Solute sites are staged ts at a time from the batch's site tables.
 // ---------------------------------------------------------------------------
-template <int LK2, int LK3, bool DIRECT, bool TCS = false>
+template <int LK2, int LK3, bool DIRECT>
 __global__ void __launch_bounds__(PlaneCfg<LK2, LK3>::NTHR, PlaneCfg<LK2, LK3>::MINB) k_pme_plane(FrameArgs a,
     int tbase, int ts, const float2* __restrict__ tab, const float* __restrict__ stn,
     const float* __restrict__ engfacT, const float2* __restrict__ fft_tw, float2* __restrict__ Y,
-    double* __restrict__ partial, int* __restrict__ errflags) {
+    double* __restrict__ partial) {
   using C = PlaneCfg<LK2, LK3>;
   constexpr int K2 = C::K2, K3 = C::K3, PITCH = C::PITCH, E = C::E, NTHR = C::NTHR;
   extern __shared__ __align__(16) unsigned char psm[];
@@ -488,13 +544,7 @@ __global__ void __launch_bounds__(PlaneCfg<LK2, LK3>::NTHR, PlaneCfg<LK2, LK3>::
   float2 acc[E];
 #pragma unroll
   for (int e = 0; e < E; ++e) acc[e] = make_float2(0.f, 0.f);
-  if constexpr (TCS) {
-    static_assert(DIRECT && K2 == K3 && K2 == 128, "tensor-core site sums here: 128 x 128 planes (k_pme_plane_pair: 64)");
-    __shared__ __align__(8) uint64_t tcs_bar;
-    __shared__ uint32_t tcs_tmem;
-    unsigned char* opnd = (unsigned char*)(((uintptr_t)plane + 1023) & ~(uintptr_t)1023);
-    tcs::site_sums<K2, E, NTHR>(tab, pair0, s, nk, Kh1, k1, k30, opnd, &tcs_bar, &tcs_tmem, errflags, acc);
-  } else if (!DIRECT && C::FIXED) {
+  if (!DIRECT && C::FIXED) {
     // q_a B1_a(k1) w2 w3 scattered on the (n2, n3) plane: a thread per (site, stencil point),
     // integer atomics in 2^-40 fixed point (exact, order-independent), real then imaginary part
     constexpr double kFix = 1099511627776.0, kUnfix = 1.0 / 1099511627776.0;
@@ -735,6 +785,182 @@ __global__ void __launch_bounds__(2 << LK, 3) k_pme_plane_pair(FrameArgs a, int 
   grid_dep_wait();
 }
 
+// ---------------------------------------------------------------------------
+// k_pme_plane128: one 128 x 128 plane a CTA of 512 threads, direct site sums on the tensor cores
+// (site_mma128).  Each axis is the radix 8, 4, 4 transform of fft_stages with the same butterflies
+// and twiddles, so the same roundings, but with the last two stages of a line's 16 points
+// {k + 8 m} in one thread's registers: a line then crosses shared memory once between its first
+// stage and the rest, not twice per stage.
+//   thread (k2, q) takes k3 = 32 q .. of column k2 from TMEM, applies G and stores them;
+//   rows (k2 -> n2): a warp owns eight rows k3; its exchange stays inside the row (position
+//     9 (p / 8) + p mod 8 and rows of 152 points: free of bank conflicts);
+//   columns (k3 -> n3): thread (n2, q) does the first-stage butterflies 4 q + i, exchanges through the
+//     same array, finishes the points of k = 2 q, 2 q + 1 and stores them as 256-byte rows of Y.
+// The plane crosses shared memory eight times where the stage by stage transform took fourteen.
+// Measured on the 60-site chain, 2048 insertions into 32,768 waters (52 planes, four tiles of sites):
+// the plane stage 21.5 -> 16.4 ms a frame, the frame 40.1 -> 35.1 ms.  With one CTA an SM (200 KB), its
+// phases follow one another: issue slots 46 % busy, shared memory 48 %, tensor pipe 15 %.
+// ---------------------------------------------------------------------------
+constexpr int kRowPitch128 = 152;
+
+// The last two radix-4 stages of a 128-point inverse transform for the 16 points p = k + 8 m (w[m]):
+// on return w[4 r2 + r3] is output 8 r2 + k + 32 r3.  tw[m] = exp(-2 pi i m / 128).
+__device__ __forceinline__ float2 untwiddle(float2 x, float2 w) {
+  return make_float2(x.x * w.x + x.y * w.y, x.y * w.x - x.x * w.y);
+}
+__device__ __forceinline__ void idft128_tail(float2 (&w)[16], const float2 (&t2)[3], const float2 (&t3)[12]) {
+  float2 o[4][4];
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    float2 v[4] = {w[a], untwiddle(w[a + 4], t2[0]), untwiddle(w[a + 8], t2[1]), untwiddle(w[a + 12], t2[2])};
+    dft<4, true>(v);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) o[a][r] = v[r];
+  }
+#pragma unroll
+  for (int r2 = 0; r2 < 4; ++r2) {
+    float2 v[4] = {o[0][r2], untwiddle(o[1][r2], t3[3 * r2]), untwiddle(o[2][r2], t3[3 * r2 + 1]),
+                   untwiddle(o[3][r2], t3[3 * r2 + 2])};
+    dft<4, true>(v);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) w[4 * r2 + r] = v[r];
+  }
+}
+__device__ __forceinline__ void tail_twiddles(const float2* tw, int k, float2 (&t2)[3], float2 (&t3)[12]) {
+#pragma unroll
+  for (int r = 1; r < 4; ++r) {
+    t2[r - 1] = tw[(k * r) << 2];
+#pragma unroll
+    for (int r2 = 0; r2 < 4; ++r2) t3[3 * r2 + r - 1] = tw[(8 * r2 + k) * r];
+  }
+}
+
+__global__ void __launch_bounds__(512, 1) k_pme_plane128(FrameArgs a, int tbase, const float2* __restrict__ tab,
+    const float* __restrict__ engfacT, const float2* __restrict__ fft_tw, float2* __restrict__ Y,
+    double* __restrict__ partial, int* __restrict__ errflags) {
+  constexpr int K = 128, RP = kRowPitch128;
+  extern __shared__ __align__(16) unsigned char psm[];
+  const int k1 = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int K1 = a.K1, Kh1 = a.Kh1, s = a.nsite, nk = Kh1 + 2 * K;
+  float2* tw2 = (float2*)psm;                              // [K] of K2, then [K] of K3
+  float2* tw3 = tw2 + K;
+  unsigned char* opnd = (unsigned char*)(((uintptr_t)(tw3 + K) + 1023) & ~(uintptr_t)1023);
+  float2* A = (float2*)opnd;                               // the plane, rows of RP points, over the dead operands
+  __shared__ __align__(8) uint64_t bars[2];
+  __shared__ uint32_t tcs_tmem;
+  for (int p = tid; p < 2 * K; p += 512) tw2[p] = fft_tw[K1 + p];
+  const int col = (warp & 3) * 32 + lane, q = warp >> 2;   // TMEM lane quarter of this warp
+  float g[32];                                             // G of this thread's points, fetched during the staging
+  {
+    const float* gk = engfacT + ((size_t)k1 * K + 32 * q) * K + col;
+#pragma unroll
+    for (int e = 0; e < 32; ++e) g[e] = __ldg(gk + (size_t)e * K);
+  }
+  const uint32_t tmem = tcs::site_mma128(tab, (size_t)(tbase + b) * s, k1, s, nk, Kh1, opnd, bars, &tcs_tmem, errflags);
+  double self = 0.0;
+  {
+#pragma unroll
+    for (int c = 0; c < 32; c += 8) {
+      uint32_t x[2][8];
+      const uint32_t t = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(2 * (32 * q + c));
+      tc::tmem_ld8(t, x[0]);
+      tc::tmem_ld8(t + 8, x[1]);
+      tc::tmem_ld_wait();
+      // influence function and the plane's share of the self energy (recpcal.F90:482-497);
+      // each mode's G |Qhat|^2 is formed in FP32 (~1e-7 relative) and summed in FP64
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float xr = __uint_as_float(x[e >> 2][2 * (e & 3)]), xi = __uint_as_float(x[e >> 2][2 * (e & 3) + 1]);
+        self += (double)(g[c + e] * (xr * xr + xi * xi));
+        A[(32 * q + c + e) * RP + col] = make_float2(xr * g[c + e], xi * g[c + e]);
+      }
+    }
+  }
+  if (k1 == 0 || 2 * k1 == K1) self *= 0.5;
+  tcs::tmem_release<K>(tmem);                              // also: the plane is in shared memory
+  float2 v[4][8], w[2][16];
+  {
+    // rows k3 = 8 warp ..: first stage, lane (row parity, j)
+    float2* R = A + (size_t)(8 * warp + (lane >> 4)) * RP;
+    const int j = lane & 15;
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+#pragma unroll
+      for (int r = 0; r < 8; ++r) v[t][r] = R[2 * t * RP + j + 16 * r];
+    __syncwarp();
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      dft<8, true>(v[t]);
+#pragma unroll
+      for (int r = 0; r < 8; ++r) R[2 * t * RP + 9 * j + r] = v[t][r];
+    }
+    __syncwarp();
+  }
+  {
+    // the other two, lane (row, k)
+    const int k = lane & 7;
+    float2* R = A + (size_t)(8 * warp + (lane >> 3)) * RP + k;
+    float2 t2[3], t3[12];
+    tail_twiddles(tw2, k, t2, t3);
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int m = 0; m < 16; ++m) w[h][m] = R[4 * h * RP + 9 * m];
+    __syncwarp();
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      idft128_tail(w[h], t2, t3);
+#pragma unroll
+      for (int r2 = 0; r2 < 4; ++r2)
+#pragma unroll
+        for (int r3 = 0; r3 < 4; ++r3) R[4 * h * RP + 8 * r2 + 32 * r3] = w[h][4 * r2 + r3];
+    }
+  }
+  __syncthreads();
+  // columns
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int r = 0; r < 8; ++r) v[i][r] = A[(4 * q + i + 16 * r) * RP + col];
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    dft<8, true>(v[i]);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) A[(8 * (4 * q + i) + r) * RP + col] = v[i][r];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int m = 0; m < 16; ++m) w[h][m] = A[(2 * q + h + 8 * m) * RP + col];
+  grid_dep_launch();                                       // the k1 transform may start filling the tail
+  float2* y = Y + ((size_t)b * Kh1 + k1) * K * K + col;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    float2 t2[3], t3[12];
+    tail_twiddles(tw3, 2 * q + h, t2, t3);
+    idft128_tail(w[h], t2, t3);
+#pragma unroll
+    for (int r2 = 0; r2 < 4; ++r2)
+#pragma unroll
+      for (int r3 = 0; r3 < 4; ++r3) y[(size_t)(8 * r2 + 2 * q + h + 32 * r3) * K] = w[h][4 * r2 + r3];
+  }
+  // the plane's share of the self energy, reduced in a fixed order; the k1 transform sums
+  // the planes of each target (self_energy_sum)
+  __shared__ double red[16];
+  self = warp_sum(self);
+  if (lane == 0) red[warp] = self;
+  __syncthreads();
+  if (warp == 0) {
+    const double t = warp_sum(lane < 16 ? red[lane] : 0.0);
+    if (lane == 0) partial[(size_t)b * Kh1 + k1] = t;
+  }
+  // Launched behind the previous chunk's gather, which reads the potential grid that this
+  // chunk's k1 transform overwrites: this grid does not complete before that gather has.
+  grid_dep_wait();
+}
+
 // selfrec[base + b] = sum over the planes k1 <= k1max of target b's shares, in
 // plane order.  Run by the first CTA of the k1 transform: every plane of the
 // chunk is complete by then.
@@ -961,12 +1187,10 @@ size_t plane_smem(const FrameArgs& a, bool direct) {
   return sizeof(float2) * (size_t)(a.K2 + a.K3) + sizeof(float2) * (size_t)a.K3 * (a.K2 + 1) + tile;
 }
 
-// the tensor-core site-sum variant (64 x 64 planes): twiddles, then the plane or the TF32
-// operands aliased over it, 1024-byte aligned
-template <int KN>
-size_t plane_smem_tcs() {
-  const size_t plane = sizeof(float2) * KN * (KN + 1);
-  return sizeof(float2) * 2 * KN + 1024 + std::max(plane, (size_t)tcs::Shape<KN>::kOperandBytes);
+// k_pme_plane128: twiddles, then two operand buffers or the plane aliased over them, 1024-byte aligned
+size_t plane_smem_128() {
+  return sizeof(float2) * 256 + 1024 + std::max(sizeof(float2) * 128 * (size_t)kRowPitch128,
+                                                2 * (size_t)tcs::Shape<128>::kOperandBytes);
 }
 
 // k_pme_plane_pair<LK>: the TF32 operands and, aliased over them, the two planes' K (K + 1)
@@ -992,7 +1216,7 @@ cudaError_t plane_attr(const FrameArgs& a) {
   cudaError_t e = raise_smem_limit(k_pme_plane<L2, L3, true>, plane_smem(a, true));
   if (e == cudaSuccess) e = raise_smem_limit(k_pme_plane<L2, L3, false>, plane_smem(a, false));
   if constexpr (L2 == 7 && L3 == 7)
-    if (e == cudaSuccess) e = raise_smem_limit(k_pme_plane<L2, L3, true, true>, plane_smem_tcs<(1 << L2)>());
+    if (e == cudaSuccess) e = raise_smem_limit(k_pme_plane128, plane_smem_128());
   if constexpr (L2 == 6 && L3 == 6)
     if (e == cudaSuccess) e = raise_smem_limit(k_pme_plane_pair<6>, plane_smem_pair<6>());
   return e;
@@ -1015,20 +1239,19 @@ void plane_launch(const FrameArgs& a, const DeviceState& d, int tbase, int nb, b
   }
   if constexpr (L2 == 7 && L3 == 7) {
     if (direct && a.nsite <= tcs::kMaxSites) {   // site sums on the tensor cores
-      launch_k(pdl, grid, C::NTHR, plane_smem_tcs<(1 << L2)>(), s, k_pme_plane<L2, L3, true, true>, a, tbase, ts,
-               (const float2*)d.sitetab, (const float*)d.sitestn, (const float*)d.engfacT,
-               (const float2*)d.fft_tw, d.spec, d.partial, err);
+      launch_k(pdl, grid, 512, plane_smem_128(), s, k_pme_plane128, a, tbase, (const float2*)d.sitetab,
+               (const float*)d.engfacT, (const float2*)d.fft_tw, d.spec, d.partial, err);
       return;
     }
   }
   if (direct)
     launch_k(pdl, grid, C::NTHR, plane_smem(a, true), s, k_pme_plane<L2, L3, true>, a, tbase, ts,
              (const float2*)d.sitetab, (const float*)d.sitestn, (const float*)d.engfacT, (const float2*)d.fft_tw,
-             d.spec, d.partial, err);
+             d.spec, d.partial);
   else
     launch_k(pdl, grid, C::NTHR, plane_smem(a, false), s, k_pme_plane<L2, L3, false>, a, tbase, ts,
              (const float2*)d.sitetab, (const float*)d.sitestn, (const float*)d.engfacT, (const float2*)d.fft_tw,
-             d.spec, d.partial, err);
+             d.spec, d.partial);
 }
 }  // namespace
 
