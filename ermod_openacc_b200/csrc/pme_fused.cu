@@ -24,7 +24,8 @@
 //                   into the insertion-fastest potential layout the gather
 //                   reads: n1 pairs (phi(2m), phi(2m+1)) per target, 32
 //                   targets, for each line n3*K2 + n2
-//                   (K1 <= 64; k_pme_rows does K1 = 128 in shared memory).
+//                   (K1 <= 64; k_pme_lines128 does K1 = 128, k_pme_lines_few
+//                   chunks of few targets).
 //
 // The FFTs are radix-8/4 Stockham stages (Govindaraju et al., "High
 // performance discrete Fourier transforms on graphics processors", SC08):
@@ -115,7 +116,6 @@ __device__ __forceinline__ void fft_batch(float2* buf, const float2* __restrict_
 constexpr int kSiteTile = 32;                  // solute sites staged in shared memory at a time (at most)
 constexpr int kTabPairs = 8;                   // (target, site) pairs per CTA of k_site_tables
 constexpr int kStn = 2 + 2 * kMaxOrder;        // stencil record: g2, g3, w2[kMaxOrder], w3[kMaxOrder]
-constexpr int kRowThreads = 512;
 constexpr int kLineRows = 4;                   // n2 rows per CTA of k_pme_lines (a warp each): 4 or 8
 constexpr int kLoadBatch = 8;                  // global loads a thread keeps in flight while staging
 
@@ -805,9 +805,6 @@ constexpr int kRowPitch128 = 152;
 
 // The last two radix-4 stages of a 128-point inverse transform for the 16 points p = k + 8 m (w[m]):
 // on return w[4 r2 + r3] is output 8 r2 + k + 32 r3.  tw[m] = exp(-2 pi i m / 128).
-__device__ __forceinline__ float2 untwiddle(float2 x, float2 w) {
-  return make_float2(x.x * w.x + x.y * w.y, x.y * w.x - x.x * w.y);
-}
 __device__ __forceinline__ void idft128_tail(float2 (&w)[16], const float2 (&t2)[3], const float2 (&t3)[12]) {
   float2 o[4][4];
 #pragma unroll
@@ -974,83 +971,7 @@ __device__ __forceinline__ void self_energy_sum(const FrameArgs& a, int base, in
 }
 
 // ---------------------------------------------------------------------------
-// k_pme_rows<LM>: grid (K3, K2 / G2), kRowThreads threads, G2 = 256 / M rows
-// of n2 for all 32 targets; M = K1 / 2 = 2^LM.  Shared rows k1 = 0..M hold
-// Y[b][k1][n3][n2] at column (n2 - n2g) * 33 + b.
-// ---------------------------------------------------------------------------
-template <int LM>
-__global__ void __launch_bounds__(kRowThreads, 2) k_pme_rows(FrameArgs a, int base, int nb, const float2* __restrict__ Y,
-    const float2* __restrict__ fft_tw, const double* __restrict__ partial, double* __restrict__ selfrec,
-    float* __restrict__ phi) {
-  constexpr int M = 1 << LM, K1 = 2 * M, Kh1 = M + 1;
-  constexpr int G2 = 256 / M, LG2 = 8 - LM, T = 32 * G2, LT = LG2 + 5, TP = G2 * 33;
-  extern __shared__ __align__(16) unsigned char rsm[];
-  const int K2 = a.K2, K3 = a.K3;
-  const int n3 = blockIdx.x, n2g = blockIdx.y * G2;
-  const int tid = threadIdx.x;
-  grid_dep_wait();
-  self_energy_sum(a, base, nb, Kh1, partial, selfrec);
-  float2* twk = (float2*)rsm;          // [K1] exp(-2 pi i m / K1)
-  float2* twm = twk + K1;              // [M]  exp(-2 pi i m / M)
-  float2* S = twm + M;                 // [Kh1][TP]
-  for (int p = tid; p < K1; p += kRowThreads) twk[p] = fft_tw[p];
-  for (int p = tid; p < M; p += kRowThreads) twm[p] = fft_tw[K1 + K2 + K3 + p];
-  // stage Y with kLoadBatch independent loads in flight per thread
-  constexpr int total = T * Kh1;
-  for (int x0 = 0; x0 < total; x0 += kLoadBatch * kRowThreads) {
-    float2 v[kLoadBatch];
-    int dst[kLoadBatch];
-#pragma unroll
-    for (int u = 0; u < kLoadBatch; ++u) {
-      const int x = x0 + u * kRowThreads + tid;
-      dst[u] = -1;
-      v[u] = make_float2(0.f, 0.f);
-      if (x < total) {
-        const int j = x & (G2 - 1), r = x >> LG2;   // r = k1 * 32 + b
-        const int b = r & 31, k1 = r >> 5;
-        dst[u] = k1 * TP + j * 33 + b;
-        if (b < nb && k1 <= a.k1max) v[u] = Y[(((size_t)b * Kh1 + k1) * K3 + n3) * K2 + n2g + j];
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < kLoadBatch; ++u)
-      if (dst[u] >= 0) S[dst[u]] = v[u];
-  }
-  __syncthreads();
-  // Hermitian packing into a length-M complex sequence Z (rows 0..M-1):
-  //   Z[k] = (X[k] + conj X[M-k]) + i (X[k] - conj X[M-k]) exp(+2 pi i k / K1)
-  // so that x[2n] = Re z[n], x[2n+1] = Im z[n] for z = inverse DFT_M(Z).
-  for (int x = tid; x < T * (M / 2 + 1); x += kRowThreads) {
-    const int t = x & (T - 1), k = x >> LT;
-    const int c = (t >> 5) * 33 + (t & 31);
-    float2 xk = S[k * TP + c], xm = S[(M - k) * TP + c];
-    if (k == 0) { xk.y = 0.f; xm.y = 0.f; }
-    {
-      const float2 cm = make_float2(xm.x, -xm.y);
-      const float2 w = make_float2(twk[k].x, -twk[k].y);
-      const float2 d = cmul(csub(xk, cm), w);
-      S[k * TP + c] = make_float2(xk.x + cm.x - d.y, xk.y + cm.y + d.x);
-    }
-    if (k != 0 && 2 * k != M) {
-      const float2 ck = make_float2(xk.x, -xk.y);
-      const float2 w = make_float2(twk[M - k].x, -twk[M - k].y);
-      const float2 d = cmul(csub(xm, ck), w);
-      S[(M - k) * TP + c] = make_float2(xm.x + ck.x - d.y, xm.y + ck.y + d.x);
-    }
-  }
-  __syncthreads();
-  fft_batch<FftShape<LM, LT, 5, 33, 1, TP>, kRowThreads, true>(S, twm, tid);
-  // phi in n1 pairs: z[n] = (phi(2n), phi(2n+1)) of line (n3 K2 + n2g + j), target b
-  float2* out = (float2*)phi + ((size_t)n3 * K2 + n2g) * M * kChunk;
-  for (int x = tid; x < T * M; x += kRowThreads) {
-    const int b = x & 31, r = x >> 5;
-    const int n = r & (M - 1), j = r >> LM;
-    out[((size_t)j * M + n) * kChunk + b] = S[n * TP + j * 33 + b];
-  }
-}
-
-// ---------------------------------------------------------------------------
-// k_pme_lines<LM>: the same transform for K1 = 2M <= 64, a thread per line.
+// k_pme_lines<LM>: the k1 transform into the potential grid for K1 = 2M <= 64, a thread per line.
 // Grid (K3, K2 / kLineRows), 32 * kLineRows threads; warp j takes row
 // n2 = blockIdx.y * kLineRows + j, lane b the target.  The CTA first stages
 // the half spectra Y[b][k1][n3][n2], k1 <= k1max, of its kLineRows rows and
@@ -1131,6 +1052,78 @@ __global__ void __launch_bounds__(32 * kLineRows, 2) k_pme_lines(FrameArgs a, in
 }
 
 // ---------------------------------------------------------------------------
+// k_pme_lines128: the same for K1 = 128, grid (K3, K2 / 16, targets / 8), 128 threads: 16 rows of n2
+// of eight targets.  The half spectra of a chunk (218 MB on a 128^3 mesh) come from HBM, so what a CTA
+// reads is cut for whole 128-byte lines: 16 consecutive n2 of one (target, k1), one 16-byte load a
+// lane; it writes 64-byte runs (eight targets).  Shared layout: target b's row j at
+// b (16 LP + 2) + j LP, LP = 66: a thread reads its line in 16-byte pieces free of bank conflicts.
+// The 32-target, four-row CTAs with a staged shared-memory transform that this replaces read each line
+// of Y in four 32-byte pieces from four CTAs: 60-site chain, 2048 insertions into 32,768 waters,
+// the frame 35.1 -> 34.8 ms (16 targets of eight rows 36.1, 32 of four 38.3; the target groups are the
+// fastest grid index, so that the 64-byte runs of a line of phi meet in L2: 36.8 with them slowest).
+// ---------------------------------------------------------------------------
+constexpr int kLines128Targets = 8, kLines128Rows = 128 / kLines128Targets;
+constexpr int kLp128 = 66, kBp128 = kLines128Rows * kLp128 + 2;
+size_t lines128_smem() { return sizeof(float2) * kLines128Targets * kBp128; }
+
+__global__ void __launch_bounds__(128, 3) k_pme_lines128(FrameArgs a, int base, int nb, const float2* __restrict__ Y,
+    const __grid_constant__ Tw128 tw, const double* __restrict__ partial, double* __restrict__ selfrec,
+    float* __restrict__ phi) {
+  constexpr int M = 64, Kh1 = M + 1, NB = 8;
+  extern __shared__ __align__(16) float2 S[];
+  const int K2 = a.K2, K3 = a.K3, tid = threadIdx.x, kmax = a.k1max;
+  const int n3 = blockIdx.z, n2g = blockIdx.y * kLines128Rows, b0 = blockIdx.x * kLines128Targets;
+  const size_t plane = (size_t)K3 * K2;
+  grid_dep_wait();                                    // the planes of this chunk are complete
+  if (n3 == 0) self_energy_sum(a, base, nb, Kh1, partial, selfrec);
+  {
+    // thread (row pair q, target b, k1 parity): rows 2 q, 2 q + 1 of k1 = kp, kp + 2, ...
+    constexpr int NQ = kLines128Rows / 2;
+    static_assert(NQ * kLines128Targets == 64, "two k1 a pass");
+    const int q = tid % NQ, b = tid / NQ % kLines128Targets, kp = tid >> 6;
+    const float4* src = (const float4*)(Y + (size_t)(b0 + b) * Kh1 * plane + (size_t)n3 * K2 + n2g + 2 * q);
+    float2* dst = S + b * kBp128 + 2 * q * kLp128;
+    // two k1 a pass; NB passes' loads in flight, from a clamped (always valid) k1
+    for (int k0 = kp; k0 <= kmax; k0 += 2 * NB) {
+      float4 v[NB];
+#pragma unroll
+      for (int u = 0; u < NB; ++u) v[u] = __ldg(src + (size_t)min(k0 + 2 * u, kmax) * (plane / 2));
+#pragma unroll
+      for (int u = 0; u < NB; ++u) {
+        const int k1 = k0 + 2 * u;
+        if (k1 <= kmax) {
+          dst[k1] = make_float2(v[u].x, v[u].y);
+          dst[kLp128 + k1] = make_float2(v[u].z, v[u].w);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  grid_dep_launch();                                  // the gather may start filling the tail
+  const int b = tid % kLines128Targets, j = tid / kLines128Targets;
+  const float4* line = reinterpret_cast<const float4*>(S + b * kBp128 + j * kLp128);
+  float2 Z[M];
+#pragma unroll
+  for (int kk = 0; kk < M / 2; ++kk) {
+    const float4 w = line[kk];
+    Z[2 * kk] = 2 * kk <= kmax ? make_float2(w.x, w.y) : make_float2(0.f, 0.f);
+    Z[2 * kk + 1] = 2 * kk + 1 <= kmax ? make_float2(w.z, w.w) : make_float2(0.f, 0.f);
+  }
+  float2 xM = make_float2(0.f, 0.f);
+  if (M <= kmax) {
+    const float4 w = line[M / 2];
+    xM = make_float2(w.x, w.y);
+  }
+  hermitian_pack<6>(Z, xM, tw);
+  idft64_stages(Z, tw);
+  float2* o = (float2*)phi + (size_t)(n3 * K2 + n2g + j) * M * kChunk + b0 + b;
+#pragma unroll
+  for (int c = 0; c < 8; ++c)
+#pragma unroll
+    for (int r = 0; r < 8; ++r) o[(c + 8 * r) * kChunk] = Z[8 * c + r];
+}
+
+// ---------------------------------------------------------------------------
 // k_pme_lines_few<LM>: the same transform for chunks of at most kFewTargets targets, a thread per
 // (target, line), straight from Y (a warp's loads are a run of n2) into natural order,
 // phi[b][line][n1].  The lane-a-target kernel above does 32 targets' lines whatever their number:
@@ -1171,6 +1164,15 @@ Tw64 make_tw64() {
   return t;
 }
 
+Tw128 make_tw128() {
+  Tw128 t;
+  for (int m = 0; m < 128; ++m) {
+    const double ang = 2.0 * kPi * (double)m / 128.0;
+    t.w[m] = make_float2((float)std::cos(ang), (float)-std::sin(ang));
+  }
+  return t;
+}
+
 bool pow2_in(int k, int lo, int hi) { return k >= lo && k <= hi && (k & (k - 1)) == 0; }
 int lg(int k) { int l = 0; while ((1 << l) < k) ++l; return l; }
 
@@ -1200,11 +1202,6 @@ size_t plane_smem_pair() {
   constexpr int K = 1 << LK;
   const size_t rows = sizeof(float2) * (size_t)(2 * K * (K + 1));
   return 1024 + std::max(rows, (size_t)tcs::Shape<K>::kOperandBytes);
-}
-
-size_t rows_smem(const FrameArgs& a) {
-  const int M = a.K1 / 2, G2 = 256 / M;
-  return sizeof(float2) * (size_t)(a.K1 + M) + sizeof(float2) * (size_t)a.Kh1 * G2 * 33;
 }
 
 // Compile-time plane sizes: every (K2, K3) in {16..128}^2 with K2 K3 >= 512.
@@ -1258,11 +1255,10 @@ void plane_launch(const FrameArgs& a, const DeviceState& d, int tbase, int nb, b
 bool fused_supported(const FrameArgs& a) {
   if (!a.pme) return false;
   if (!pow2_in(a.K1, 16, 128) || !pow2_in(a.K2, 16, 128) || !pow2_in(a.K3, 16, 128)) return false;
-  const int M = a.K1 / 2, G2 = 256 / M;
-  if (G2 > a.K2) return false;                       // one CTA of k_pme_rows spans G2 rows of n2
+  if (256 / (a.K1 / 2) > a.K2) return false;         // 16 x 16 planes at K1 = 16 stay on the cuFFT path
   if (a.K2 * a.K3 < 512) return false;               // at least 32 threads per plane
   if (a.K3 % plane_elems(a) != 0) return false;      // a thread owns E consecutive k3
-  return plane_smem(a, true) <= 220 * 1024 && plane_smem(a, false) <= 220 * 1024 && rows_smem(a) <= 220 * 1024;
+  return plane_smem(a, true) <= 220 * 1024 && plane_smem(a, false) <= 220 * 1024;
 }
 
 int setup_fused(const FrameArgs& a) {
@@ -1274,11 +1270,10 @@ int setup_fused(const FrameArgs& a) {
 #undef ERM_ATTR
   if (e != cudaSuccess) return -1;
   const int lm = lg(a.K1 / 2);
-  const int sm = (int)rows_smem(a);
   if (lm == 3) e = raise_smem_limit(k_pme_lines<3>, lines_smem(8));
   if (lm == 4) e = raise_smem_limit(k_pme_lines<4>, lines_smem(16));
   if (lm == 5) e = raise_smem_limit(k_pme_lines<5>, lines_smem(32));
-  if (lm == 6) e = raise_smem_limit(k_pme_rows<6>, (size_t)sm);
+  if (lm == 6) e = raise_smem_limit(k_pme_lines128, lines128_smem());
   return e == cudaSuccess ? 0 : -1;
 }
 
@@ -1345,12 +1340,9 @@ void launch_pme_rows(const FrameArgs& a, const DeviceState& d, int base, int nb,
       return;
     default: break;
   }
-  const int M = a.K1 / 2, G2 = 256 / M;
-  const dim3 grid(a.K3, a.K2 / G2);
-  const size_t sm = rows_smem(a);
-  switch (lg(M)) {
-    default: k_pme_rows<6><<<grid, kRowThreads, sm, s>>>(a, base, nb, d.spec, d.fft_tw, d.partial, d.selfrec, d.phi); break;
-  }
+  static const Tw128 t128 = make_tw128();
+  launch_k(pdl, dim3((nb + kLines128Targets - 1) / kLines128Targets, a.K2 / kLines128Rows, a.K3), 128, lines128_smem(), s,
+           k_pme_lines128, a, base, nb, (const float2*)d.spec, t128, (const double*)d.partial, d.selfrec, d.phi);
 }
 
 }  // namespace erm

@@ -65,11 +65,49 @@ struct Tw64 {
   float2 w[64];
 };
 
-// exp(+2 pi i m / N) for N dividing 64
+// the same for lengths up to 128
+struct Tw128 {
+  float2 w[128];
+};
+
+// exp(+2 pi i m / N) for N dividing the table's length
 template <int N>
 ERM_HD float2 wplus(const Tw64& t, int m) {
   static_assert(N >= 1 && N <= 64 && (64 % N) == 0, "N divides 64");
   return conj(t.w[(m & (N - 1)) * (64 / N)]);
+}
+template <int N>
+ERM_HD float2 wplus(const Tw128& t, int m) {
+  static_assert(N >= 1 && N <= 128 && (128 % N) == 0, "N divides 128");
+  return conj(t.w[(m & (N - 1)) * (128 / N)]);
+}
+
+// x times the conjugate of w
+ERM_HD float2 untwiddle(float2 x, float2 w) {
+  return make_float2(x.x * w.x + x.y * w.y, x.y * w.x - x.x * w.y);
+}
+
+// In-register inverse DFT of length 64 as two radix-8 stages, outputs in order, with the butterflies,
+// twiddles and roundings of the staged shared-memory transform of the same length.
+ERM_HD void idft64_stages(float2 (&Z)[64], const Tw128& t) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    float2 v[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) v[r] = Z[j + 8 * r];
+    dft<8, true>(v);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) Z[j + 8 * r] = v[r];       // first-stage output 8 j + r, kept at j + 8 r
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    float2 v[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) v[r] = r == 0 ? Z[8 * j] : untwiddle(Z[8 * j + r], t.w[2 * j * r]);
+    dft<8, true>(v);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) Z[8 * j + r] = v[r];       // output j + 8 r, kept at 8 j + r
+  }
 }
 
 // In-register inverse DFT of length M = 2^LM, 3 <= LM <= 5:
@@ -137,8 +175,8 @@ ERM_HD void idft64_reg(float2 (&Z)[64], const Tw64& t) {
 //   Z[k] = (X[k] + conj X[M-k]) + i (X[k] - conj X[M-k]) exp(+2 pi i k / K1),
 // so that for z = inverse DFT_M(Z), x[2n] = Re z[n] and x[2n+1] = Im z[n] is
 // the inverse real DFT of length K1.  Z holds X[0..M-1] on entry, xM = X[M].
-template <int LM>
-ERM_HD void hermitian_pack(float2 (&Z)[1 << LM], float2 xM, const Tw64& t) {
+template <int LM, class Tw>
+ERM_HD void hermitian_pack(float2 (&Z)[1 << LM], float2 xM, const Tw& t) {
   constexpr int M = 1 << LM, K1 = 2 * M;
 #pragma unroll
   for (int k = 0; k <= M / 2; ++k) {
