@@ -241,12 +241,30 @@ __device__ __forceinline__ uint32_t tf32_bits(float x) {
 __device__ __forceinline__ uint32_t* slot(unsigned char* tile, int row, int k) {
   return (uint32_t*)(tile + tc::swz(row, k >> 2)) + (k & 3);
 }
+// The two TF32 terms of v.  The high one is rounded (to nearest, ties away from zero) by integer
+// arithmetic: conversions run at a quarter of the rate and bounded the staging.  A NaN may lose its
+// high term to the carry, but not the low one, v - hi.
+struct Split {
+  uint32_t hi, lo;
+};
+__device__ __forceinline__ Split split(float v) {
+  const uint32_t h = (__float_as_uint(v) + 0x1000u) & 0xffffe000u;
+  return {h, tf32_bits(v - __uint_as_float(h))};
+}
+__device__ __forceinline__ Split neg(Split v) { return {v.hi ^ 0x80000000u, v.lo ^ 0x80000000u}; }
 // the pair (v0, v1) at columns (k, k + 1), k even: one 8-byte store into each of hi and lo
+__device__ __forceinline__ void put2(unsigned char* hi, unsigned char* lo, int row, int k, Split v0, Split v1) {
+  *reinterpret_cast<uint2*>(slot(hi, row, k)) = make_uint2(v0.hi, v1.hi);
+  *reinterpret_cast<uint2*>(slot(lo, row, k)) = make_uint2(v0.lo, v1.lo);
+}
 __device__ __forceinline__ void put_split2(unsigned char* hi, unsigned char* lo, int row, int k, float v0, float v1) {
-  const uint32_t h0 = tf32_bits(v0), h1 = tf32_bits(v1);
-  *reinterpret_cast<uint2*>(slot(hi, row, k)) = make_uint2(h0, h1);
-  *reinterpret_cast<uint2*>(slot(lo, row, k)) =
-      make_uint2(tf32_bits(v0 - __uint_as_float(h0)), tf32_bits(v1 - __uint_as_float(h1)));
+  put2(hi, lo, row, k, split(v0), split(v1));
+}
+// rows (2 c, 2 c + 1) of B: (Re, -Im) and (Im, Re)
+__device__ __forceinline__ void put_b(unsigned char* hi, unsigned char* lo, int c, int k, float2 v) {
+  const Split x = split(v.x), y = split(v.y);
+  put2(hi, lo, 2 * c, k, x, neg(y));
+  put2(hi, lo, 2 * c + 1, k, y, x);
 }
 __device__ __forceinline__ void mma(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
   const uint32_t z = 0;
@@ -258,129 +276,88 @@ __device__ __forceinline__ void mma(uint32_t tmem_d, uint64_t da, uint64_t db, u
       : "r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(z), "r"(z), "r"(z), "r"(z));
 }
 
-// The staging, MMAs and bounded wait of site_sums; returns the TMEM address of the product,
-// which the caller reads and then frees with tmem_release.  Rows 0..KN-1 of A hold D_s(k2) of
-// plane k1A of the target whose site tables start at pairA.  KN = 64: rows 64..127 hold those
-// of plane k1B of the target at pairB (zero when k1B < 0).  Two targets take two rounds, each
-// with its own B3 and the other half's A rows zero, accumulating in the same TMEM columns.
-template <int KN, int NTHR>
-__device__ uint32_t site_mma(const float2* __restrict__ tab, size_t pairA, int k1A, size_t pairB, int k1B, int s,
-                             int nk, int Kh1, unsigned char* opnd, uint64_t* bar, uint32_t* tmem_slot,
-                             int* __restrict__ errflags) {
+// The product of k_pme_plane_pair (64 x 64 planes, two a CTA, 128 threads): staging, MMAs and bounded
+// wait; returns the TMEM address of the product, which the caller reads and then frees with
+// tmem_release.  Rows 0..63 of A hold D_s(k2) of plane k1A of the target whose site tables start at
+// pairA, rows 64..127 those of plane k1B of the target at pairB (zero when k1B < 0).  Two targets take
+// two rounds, each with its own B3 and the other half's A rows zero, accumulating in the same TMEM
+// columns.  A CTA's staging is a chain of waits that nothing else hides (at most three CTAs an SM,
+// in step): every table value of a tile is in flight at once, the next tile's during the products,
+// and meanwhile() (the fetch of G) runs once the last tile is staged.
+template <class F>
+__device__ __forceinline__ uint32_t site_mma64(const float2* __restrict__ tab, size_t pairA, int k1A, size_t pairB,
+                                               int k1B, int s, int nk, int Kh1, unsigned char* opnd, uint64_t* bar,
+                                               uint32_t* tmem_slot, int* __restrict__ errflags, F meanwhile) {
+  constexpr int KN = 64, NTHR = 128, NI = kTileSites * KN / NTHR;
   using Sh = Shape<KN>;
   using namespace tc;
-  constexpr int NI = kTileSites * KN / NTHR;           // staging items of a thread per loop, full tile
-  static_assert(NI * NTHR == kTileSites * KN, "whole items per thread");
-  constexpr int NB = NI < 4 ? NI : 4;                   // items loaded together (registers)
-  const int tid = threadIdx.x, warp = tid >> 5;
-  unsigned char* ahi = opnd;
-  unsigned char* alo = ahi + Sh::kAB;
-  unsigned char* bhi = alo + Sh::kAB;
-  unsigned char* blo = bhi + Sh::kBB;
-  if (warp == 0) {
+  const int tid = threadIdx.x;
+  // first: an SM starts its next CTA of such a kernel only once this one has given up the permit
+  if (tid < 32) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                  "r"(Sh::kTmemCols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
+  unsigned char* ahi = opnd;
+  unsigned char* alo = ahi + Sh::kAB;
+  unsigned char* bhi = alo + Sh::kAB;
+  unsigned char* blo = bhi + Sh::kBB;
+  // The item orders put the 16 lanes of a half warp on 16 distinct (16-byte chunk, half) slots of the
+  // swizzled rows, so the 8-byte stores are free of bank conflicts: a lane's chunk is (t / 2) ^ (row
+  // mod 8), its half t mod 2.
+  // A item u: row k2 = qa, site ta + 2 u; B item u: rows of k3 = qb + 32 (u mod 2), site tb + 4 (u / 2)
+  const int qa = (tid & 7) | (((tid >> 4) & 7) << 3), ta = (tid >> 3) & 1;
+  const int qb = (tid & 3) | (((tid >> 4) & 7) << 2), tb = (tid >> 2) & 3;
+  const bool cross = k1B >= 0 && pairB != pairA;
+  const int tiles = (s + kTileSites - 1) / kTileSites, total = cross ? 2 * tiles : tiles;
+  float2 cA[NI], cB[NI], b2[NI], b3[NI];
+  auto load = [&](int tile) {                          // tile of a round: sites past s are zeros
+    const bool second = tile >= tiles;
+    const int t0 = (second ? tile - tiles : tile) * kTileSites;
+    const bool onA = !second, onB = k1B >= 0 && (second || !cross);
+    const float2* base = tab + (second ? pairB : pairA) * nk;
+#pragma unroll
+    for (int u = 0; u < NI; ++u) {
+      const int t = t0 + ta + 2 * u, v = t0 + tb + 4 * (u >> 1);
+      cA[u] = cB[u] = b2[u] = b3[u] = make_float2(0.f, 0.f);
+      if (t < s) {
+        const float2* row = base + (size_t)t * nk;
+        if (onA) cA[u] = __ldg(row + k1A);
+        if (onB) cB[u] = __ldg(row + k1B);
+        b2[u] = __ldg(row + Kh1 + qa);
+      }
+      if (v < s) b3[u] = __ldg(base + (size_t)v * nk + Kh1 + KN + qb + 32 * (u & 1));
+    }
+  };
+  load(0);
   if (tid == 0) {
     mbar_init(bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   bool ok = true;
   uint32_t tmem = 0;                                   // read once the first tile's barrier has passed (s >= 1)
-  int tile = 0;
-  const bool cross = KN == 64 && k1B >= 0 && pairB != pairA;
-  for (int round = 0; round < (cross ? 2 : 1); ++round)
-  for (int t0 = 0; t0 < s && ok; t0 += kTileSites, ++tile) {
-    const bool onA = !cross || round == 0, onB = k1B >= 0 && (!cross || round == 1);
-    const size_t pb3 = round == 0 ? pairA : pairB;    // the target whose B3 this round multiplies
-    const int ns = min(kTileSites, s - t0);
-    // K steps of 8 columns that the tile's sites fill; the columns past 2 ns of the last step are zeroed
+  for (int tile = 0; tile < total && ok; ++tile) {
+    const int ns = min(kTileSites, s - (tile >= tiles ? tile - tiles : tile) * kTileSites);
+    // K steps of 8 columns that the tile's sites fill; the columns past 2 ns of the last step are zeros
     const int nks = (2 * ns + 7) / 8;
-    if (2 * ns < 8 * nks) {
-      const int k0 = 2 * ns, k1e = 8 * nks;                 // zero columns [k0, k1e), even bounds
-      const int per = (k1e - k0) / 2;                       // column pairs a row
-      for (int x = tid; x < (kRows + Sh::kN) * per; x += NTHR) {
-        const int r = x / per, k = k0 + 2 * (x - r * per);
-        if (r < kRows) {
-          *reinterpret_cast<uint2*>(slot(ahi, r, k)) = make_uint2(0u, 0u);
-          *reinterpret_cast<uint2*>(slot(alo, r, k)) = make_uint2(0u, 0u);
-        } else {
-          *reinterpret_cast<uint2*>(slot(bhi, r - kRows, k)) = make_uint2(0u, 0u);
-          *reinterpret_cast<uint2*>(slot(blo, r - kRows, k)) = make_uint2(0u, 0u);
-        }
+#pragma unroll
+    for (int u = 0; u < NI; ++u) {
+      const int t = ta + 2 * u, v = tb + 4 * (u >> 1), k3 = qb + 32 * (u & 1);
+      if (t < 4 * nks) {
+        // q B1(k1) B2(k2 = qa); zero when off.  The roundings are fixed here, one form for each plane.
+        const float2 d = make_float2(__fmaf_rn(cA[u].x, b2[u].x, -__fmul_rn(cA[u].y, b2[u].y)),
+                                     __fmaf_rn(cA[u].y, b2[u].x, __fmul_rn(cA[u].x, b2[u].y)));
+        put_split2(ahi, alo, qa, 2 * t, d.x, d.y);
+        const float2 e = make_float2(__fmaf_rn(cB[u].x, b2[u].x, -__fmul_rn(cB[u].y, b2[u].y)),
+                                     __fmaf_rn(cB[u].x, b2[u].y, __fmul_rn(cB[u].y, b2[u].x)));
+        put_split2(ahi, alo, KN + qa, 2 * t, e.x, e.y);
+      }
+      if (v < 4 * nks) {
+        put_b(bhi, blo, k3, 2 * v, b3[u]);
       }
     }
-    // The item orders put the 16 lanes of a half warp on 16 distinct (16-byte chunk, half)
-    // slots of the swizzled rows, so the 8-byte stores are free of bank conflicts: a lane's
-    // chunk is (t / 2) ^ (row mod 8), its half t mod 2.
-    // A rows k2 = q: item bits 0-2 q mod 8, bit 3 t mod 2, bits 4.. q / 8, then t / 2.  Each
-    // loop loads NB items of the thread at a time, then splits and stores them, so that the
-    // table reads are in flight together.
-#pragma unroll 1
-    for (int u0 = 0; u0 < NI; u0 += NB) {
-      const int lim = ((ns + 1) >> 1) * 2 * KN;
-      const bool same = pairB == pairA;
-      float2 c1v[NB], b2v[NB], c1w[NB], b2w[NB];
-#pragma unroll
-      for (int u = 0; u < NB; ++u) {
-        const int x = tid + (u0 + u) * NTHR;
-        const int q = (x & 7) | (((x >> 4) & (KN / 8 - 1)) << 3);
-        const int t = ((x >> 3) & 1) | ((x / (2 * KN)) << 1);
-        const float2 z = make_float2(0.f, 0.f);
-        c1v[u] = z; b2v[u] = z; c1w[u] = z; b2w[u] = z;
-        if (x < lim && t < ns) {
-          const float2* row = tab + (pairA + t0 + t) * nk;
-          b2v[u] = row[Kh1 + q];
-          if (onA) c1v[u] = row[k1A];
-          if (KN == 64 && onB) {
-            const float2* rb = same ? row : tab + (pairB + t0 + t) * nk;
-            c1w[u] = rb[k1B];
-            if (!same) b2w[u] = rb[Kh1 + q];
-          }
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < NB; ++u) {
-        const int x = tid + (u0 + u) * NTHR;
-        const int q = (x & 7) | (((x >> 4) & (KN / 8 - 1)) << 3);
-        const int t = ((x >> 3) & 1) | ((x / (2 * KN)) << 1);
-        if (x < lim && t < ns) {
-          const float2 d = fft::cmul(c1v[u], b2v[u]);       // q B1(k1) B2(k2 = q); zero when off
-          put_split2(ahi, alo, q, 2 * t, d.x, d.y);
-          if (KN == 64) {
-            const float2 e = fft::cmul(c1w[u], same ? b2v[u] : b2w[u]);
-            put_split2(ahi, alo, 64 + q, 2 * t, e.x, e.y);
-          }
-        }
-      }
-    }
-    // B row pairs (2 c2, 2 c2 + 1): item bits 0-1 c2 mod 4, bits 2-3 t mod 4, bits 4.. c2 / 4,
-    // then t / 4.  Pair c2 holds k3 = c2.
-#pragma unroll 1
-    for (int u0 = 0; u0 < NI; u0 += NB) {
-      const int lim = ((ns + 3) >> 2) * 4 * KN;
-      float2 v[NB];
-#pragma unroll
-      for (int u = 0; u < NB; ++u) {
-        const int x = tid + (u0 + u) * NTHR;
-        const int c2 = (x & 3) | (((x >> 4) & (KN / 4 - 1)) << 2);
-        const int t = ((x >> 2) & 3) | ((x / (4 * KN)) << 2);
-        const int k3 = c2;
-        v[u] = make_float2(0.f, 0.f);
-        if (x < lim && t < ns) v[u] = tab[(pb3 + t0 + t) * nk + Kh1 + KN + k3];
-      }
-#pragma unroll
-      for (int u = 0; u < NB; ++u) {
-        const int x = tid + (u0 + u) * NTHR;
-        const int c2 = (x & 3) | (((x >> 4) & (KN / 4 - 1)) << 2);
-        const int t = ((x >> 2) & 3) | ((x / (4 * KN)) << 2);
-        if (x < lim && t < ns) {
-          put_split2(bhi, blo, 2 * c2, 2 * t, v[u].x, -v[u].y);
-          put_split2(bhi, blo, 2 * c2 + 1, 2 * t, v[u].y, v[u].x);
-        }
-      }
-    }
+    if (tile + 1 < total) load(tile + 1);
+    else meanwhile();
     fence_proxy_async();
     tc_fence_before();
     __syncthreads();
@@ -390,7 +367,7 @@ __device__ uint32_t site_mma(const float2* __restrict__ tab, size_t pairA, int k
       const uint64_t dah = smem_desc(smem_u32(ahi)), dal = smem_desc(smem_u32(alo));
       const uint64_t dbh = smem_desc(smem_u32(bhi)), dbl = smem_desc(smem_u32(blo));
       for (int ks = 0; ks < nks; ++ks)
-        mma(tmem, dah + 2 * ks, dbh + 2 * ks, Sh::kIdesc, (round > 0 || t0 > 0 || ks > 0) ? 1u : 0u);
+        mma(tmem, dah + 2 * ks, dbh + 2 * ks, Sh::kIdesc, (tile > 0 || ks > 0) ? 1u : 0u);
       for (int ks = 0; ks < nks; ++ks) mma(tmem, dah + 2 * ks, dbl + 2 * ks, Sh::kIdesc, 1u);
       for (int ks = 0; ks < nks; ++ks) mma(tmem, dal + 2 * ks, dbh + 2 * ks, Sh::kIdesc, 1u);
       mma_commit(bar);
@@ -418,7 +395,7 @@ __device__ __forceinline__ void tmem_release(uint32_t tmem) {
 
 // The 128 x 128 plane's product: one target, one plane, tiles of 16 sites in two operand buffers
 // (Shape<128>::kOperandBytes each), so that a tile is staged while the tensor cores work on the one
-// before, from table values fetched a tile ahead.  The items are ordered as site_mma's, free of bank
+// before, from table values fetched a tile ahead.  The items are ordered as site_mma64's, free of bank
 // conflicts (fetched a tile ahead, the shorter runs of table reads no longer cost what they save).
 // Bars: two mbarriers.  Returns the TMEM address of the product; 512 threads.
 __device__ __forceinline__ uint32_t site_mma128(const float2* __restrict__ tab, size_t pair0, int k1, int s, int nk,
@@ -478,8 +455,7 @@ __device__ __forceinline__ uint32_t site_mma128(const float2* __restrict__ tab, 
         put_split2(ahi, alo, qa, 2 * t, d.x, d.y);
       }
       if (v < 4 * nks) {
-        put_split2(bhi, blo, 2 * qb, 2 * v, b3[u].x, -b3[u].y);       // B3(k3 = qb)
-        put_split2(bhi, blo, 2 * qb + 1, 2 * v, b3[u].y, b3[u].x);
+        put_b(bhi, blo, qb, 2 * v, b3[u]);                    // B3(k3 = qb)
       }
     }
     load(t0 + kTileSites);
@@ -693,18 +669,33 @@ __global__ void __launch_bounds__(PlaneCfg<LK2, LK3>::NTHR, PlaneCfg<LK2, LK3>::
 
 // ---------------------------------------------------------------------------
 // k_pme_plane_pair<LK>: two planes per CTA, K x K planes (K = 2^LK = 64), 2K threads.  The
-// chunk's planes (target b, k1 <= k1max) are numbered p = b (k1max + 1) + k1 and CTA c takes
-// p = 2c and 2c + 1, so a chunk of 32 targets is at most 32 (k1max + 1) / 2 CTAs, one resident
-// wave at 3 CTAs per SM for k1max < 27.  B3 does not depend on k1, so one tensor-core product
-// serves two planes of a target: A rows 0..63 hold D(k2) of the first plane, rows 64..127
-// those of the second (zero past the chunk's last plane); a pair that spans two targets takes
-// two rounds (tcs::site_mma).  TMEM lane quarter w holds the rows that warp w reads.
+// chunk's planes (target b, k1 <= k1max) are numbered p = b (k1max + 1) + k1 and a CTA takes
+// p = 2c and 2c + 1 (c = plane_pair_of the CTA), so a chunk of 32 targets is at most
+// 32 (k1max + 1) / 2 CTAs, one resident wave at 3 CTAs per SM for k1max < 27.  B3 does not
+// depend on k1, so one tensor-core product serves two planes of a target: A rows 0..63 hold
+// D(k2) of the first plane, rows 64..127 those of the second (zero past the chunk's last
+// plane); a pair that spans two targets takes two rounds (tcs::site_mma64).  TMEM lane
+// quarter w holds the rows that warp w reads.
 // Thread (half = tid / K, k2 = tid mod K) takes all K of its column from TMEM, applies G,
-// and transforms the column in registers (idft64_reg); one transpose through shared memory
-// hands each thread a row n3 for the second axis, and the rows go back through shared
-// memory so that each warp store is one 256-byte row of Y.
-// Grid ceil(targets (k1max + 1) / 2).
+// and transforms the column in registers (idft64_reg); a transpose through shared memory
+// hands each thread a row n3 for the second axis, a second one the points of one n2, so that
+// each warp store is one 256-byte row of Y.  Grid ceil(targets (k1max + 1) / 2).
+// What bounds it is the chain of waits of a CTA, all in step.  Measured on 32 targets x 27
+// planes: 24.8 -> 20.7 us with 12 sites, 37.0 -> 28.8 us with 32 (the ring's frame 3.23 -> 3.04
+// ms) from the pairs of two targets placed first (they ended 4 us after the rest), tensor
+// memory allocated first (an SM's CTAs start one after another, each when the one before has
+// given up the permit: 3.2 -> 2.0 us for the three), the table values in flight together and
+// fewer conversions in the staging.
 // ---------------------------------------------------------------------------
+// The pair that CTA c takes.  A pair that spans two targets (kp odd: one of kp in two targets) takes
+// two rounds, so these pairs come first and do not make the launch's tail.
+__device__ __forceinline__ int plane_pair_of(int c, int kp, int nb) {
+  if ((kp & 1) == 0 || kp == 1) return c;
+  const int spans = nb / 2;
+  if (c < spans) return c * kp + (kp - 1) / 2;
+  const int j = c - spans, m = j / (kp - 1), r = j - m * (kp - 1);
+  return m * kp + r + (m < spans && r >= (kp - 1) / 2);
+}
 template <int LK>
 __global__ void __launch_bounds__(2 << LK, 3) k_pme_plane_pair(FrameArgs a, int tbase, int nb,
     const float2* __restrict__ tab, const float* __restrict__ engfacT, Tw64 t64, float2* __restrict__ Y,
@@ -714,7 +705,7 @@ __global__ void __launch_bounds__(2 << LK, 3) k_pme_plane_pair(FrameArgs a, int 
   extern __shared__ __align__(16) unsigned char psm[];
   const int tid = threadIdx.x, warp = tid >> 5;
   const int half = tid >> LK, i = tid & (K - 1);          // plane of the pair; column k2, later row n3
-  const int kp = a.k1max + 1, p0 = 2 * blockIdx.x;
+  const int kp = a.k1max + 1, p0 = 2 * plane_pair_of(blockIdx.x, kp, nb);
   const bool has1 = p0 + 1 < nb * kp;
   const int b0 = p0 / kp, k1a = p0 - b0 * kp;
   const int b1 = has1 ? (p0 + 1) / kp : b0, k1b = has1 ? p0 + 1 - b1 * kp : -1;
@@ -723,21 +714,20 @@ __global__ void __launch_bounds__(2 << LK, 3) k_pme_plane_pair(FrameArgs a, int 
   const int Kh1 = a.Kh1, s = a.nsite, nk = Kh1 + 2 * K;
   unsigned char* opnd = (unsigned char*)(((uintptr_t)psm + 1023) & ~(uintptr_t)1023);
   float2* xp = (float2*)opnd + half * K * P;              // this plane's [n][P], over the dead operands
-  float gv[K];                                            // G of column k2, prefetched during the staging
-  {
-    const float* gk = engfacT + (size_t)k1 * K * K + i;
-#pragma unroll
-    for (int e = 0; e < K; ++e) gv[e] = gk[(size_t)e * K];
-  }
+  float gv[K];                                            // G of column k2, fetched during the products
   __shared__ __align__(8) uint64_t tcs_bar;
   __shared__ uint32_t tcs_tmem;
   const uint32_t tmem =
-      tcs::site_mma<K, NTHR>(tab, (size_t)(tbase + b0) * s, k1a, (size_t)(tbase + b1) * s, k1b, s, nk, Kh1,
-                             opnd, &tcs_bar, &tcs_tmem, errflags);
+      tcs::site_mma64(tab, (size_t)(tbase + b0) * s, k1a, (size_t)(tbase + b1) * s, k1b, s, nk, Kh1, opnd, &tcs_bar,
+                      &tcs_tmem, errflags, [&]() {
+                        const float* gk = engfacT + (size_t)k1 * K * K + i;
+#pragma unroll
+                        for (int e = 0; e < K; ++e) gv[e] = __ldg(gk + (size_t)e * K);
+                      });
   // influence function and the plane's share of the self energy (recpcal.F90:482-497);
   // each mode's G |Qhat|^2 is formed in FP32 (~1e-7 relative) and summed in FP64
   float2 z[K];
-  double self = 0.0;
+  double part[4] = {0.0, 0.0, 0.0, 0.0};                  // four chains of FP64 adds
 #pragma unroll
   for (int c = 0; c < 2 * K; c += 32) {
     uint32_t v[32];
@@ -746,32 +736,31 @@ __global__ void __launch_bounds__(2 << LK, 3) k_pme_plane_pair(FrameArgs a, int 
     for (int j = 0; j < 16; ++j) {
       const int k3 = c / 2 + j;
       const float xr = __uint_as_float(v[2 * j]), xi = __uint_as_float(v[2 * j + 1]), g = gv[k3];
-      self += (double)(g * (xr * xr + xi * xi));
-      z[k3] = make_float2(xr * g, xi * g);
+      part[j & 3] += (double)(g * __fmaf_rn(xr, xr, __fmul_rn(xi, xi)));
+      z[k3] = make_float2(__fmul_rn(xr, g), __fmul_rn(xi, g));
     }
   }
+  double self = (part[0] + part[1]) + (part[2] + part[3]);
   if (k1 == 0 || 2 * k1 == a.K1) self *= 0.5;
   tcs::tmem_release<K>(tmem);                             // also: every thread is past the MMAs
-  idft64_reg(z, t64);                                     // column k2: n3 = 4 c + d at z[16 d + c]
+  // both axes run the same code, so that it is fetched once: column k2, then row n3
+#pragma unroll 1
+  for (int axis = 0; axis < 2; ++axis) {
+    idft64_reg(z, t64);                                   // output n = 4 c + d at z[16 d + c]
+    __syncthreads();
 #pragma unroll
-  for (int d = 0; d < 4; ++d)
+    for (int d = 0; d < 4; ++d)
 #pragma unroll
-    for (int c = 0; c < 16; ++c) xp[(4 * c + d) * P + i] = z[16 * d + c];
-  __syncthreads();
+      for (int c = 0; c < 16; ++c) xp[(4 * c + d) * P + i] = z[16 * d + c];
+    __syncthreads();
 #pragma unroll
-  for (int k2 = 0; k2 < K; ++k2) z[k2] = xp[i * P + k2];  // row n3 = i
-  idft64_reg(z, t64);                                     // n2 = 4 c + d at z[16 d + c]
-  __syncthreads();
-#pragma unroll
-  for (int d = 0; d < 4; ++d)
-#pragma unroll
-    for (int c = 0; c < 16; ++c) xp[i * P + 4 * c + d] = z[16 * d + c];
-  __syncthreads();
+    for (int k = 0; k < K; ++k) z[k] = xp[i * P + k];     // after the columns: row n3 = i; after the rows: n2 = i
+  }
   grid_dep_launch();                                      // the k1 transform may start filling the tail
   if (live) {
     float2* y = Y + ((size_t)b * Kh1 + k1) * K * K + i;
-#pragma unroll 8
-    for (int e = 0; e < K; ++e) y[(size_t)e * K] = xp[e * P + i];
+#pragma unroll
+    for (int e = 0; e < K; ++e) y[(size_t)e * K] = z[e];
   }
   // each plane's share of the self energy over its two warps, in a fixed order; the k1
   // transform sums the planes of each target (self_energy_sum)
@@ -992,7 +981,7 @@ template <int LM>
 __global__ void __launch_bounds__(32 * kLineRows, 2) k_pme_lines(FrameArgs a, int base, int nb,
     const float2* __restrict__ Y, Tw64 tw, const double* __restrict__ partial, double* __restrict__ selfrec,
     float* __restrict__ phi) {
-  constexpr int M = 1 << LM, K1 = 2 * M, Kh1 = M + 1, NT = 32 * kLineRows;
+  constexpr int M = 1 << LM, Kh1 = M + 1, NT = 32 * kLineRows;
   constexpr int LP = line_lp(M), JP = line_jp(M);
   static_assert(kLineRows == 4, "staging items: 2 row pairs x 2 k1 x 32 targets per 128 threads");
   extern __shared__ __align__(16) float2 S[];              // [kLineRows][32][LP] + pads
