@@ -1648,51 +1648,57 @@ __global__ void __launch_bounds__(kGatherThreads, 4) k_gather_rec(FrameArgs a, i
         for (int c = 0; c < 12; ++c) wl[c] = __shfl_sync(0xffffffffu, rv, src + c);
         const int off = __float_as_int(__shfl_sync(0xffffffffu, rv, src + 12));
         const int flags = __float_as_int(__shfl_sync(0xffffffffu, rv, src + 13));
-        float v[64];
-        if (!(flags & kRecWrap)) {
-          const float* p0 = phi + (size_t)off + 2 * b;
-          if (flags & kRecOdd) gather_rows4<4, true>(p0, s2, s3, 0, v);
-          else gather_rows4<4, false>(p0, s2, s3, 0, v);
-        } else if (!(flags & kRecWrapX)) {
-          // only n2 or n3 wraps: each row is contiguous in n1, loaded in pairs as above
-          const int gp = __float_as_int(__shfl_sync(0xffffffffu, rv, src + 14));
-          const int gx = gp & 1023, gy = (gp >> 10) & 1023, gz = gp >> 20;
-          const bool odd = flags & kRecOdd;
+        // two of the four stencil planes at a time: 24 loads of a lane in flight beside the sums of the
+        // two before (all 64 points first: 60-site chain, 32,768 waters, the frame 34.3 against 33.25 ms;
+        // two planes with five to seven CTAs an SM for four: 33.5, 34.1, 35.8)
 #pragma unroll
-          for (int cs = 0; cs < 4; ++cs) {
-            const int r3 = wrapk(gz - cs, K3);
+        for (int c30 = 0; c30 < 4; c30 += 2) {
+          float v[32];
+          if (!(flags & kRecWrap)) {
+            const float* p0 = phi + (size_t)off + 2 * b;
+            if (flags & kRecOdd) gather_rows4<2, true>(p0, s2, s3, c30, v);
+            else gather_rows4<2, false>(p0, s2, s3, c30, v);
+          } else if (!(flags & kRecWrapX)) {
+            // only n2 or n3 wraps: each row is contiguous in n1, loaded in pairs as above
+            const int gp = __float_as_int(__shfl_sync(0xffffffffu, rv, src + 14));
+            const int gx = gp & 1023, gy = (gp >> 10) & 1023, gz = gp >> 20;
+            const bool odd = flags & kRecOdd;
 #pragma unroll
-            for (int c2 = 0; c2 < 4; ++c2) {
-              const float* r = phi + phi_index((size_t)r3 * K2 + wrapk(gy - c2, K2), gx, b, P1);
-              float* o = v + (cs * 4 + c2) * 4;
-              if (odd) {   // pairs (gx-1, gx) and (gx-3, gx-2)
-                const float2 p = *(const float2*)(r - 1), q = *(const float2*)(r - 1 - 2 * kChunk);
-                o[0] = p.y; o[1] = p.x; o[2] = q.y; o[3] = q.x;
-              } else {     // gx alone, pair (gx-2, gx-1), gx-3 alone
-                const float2 p = *(const float2*)(r - 2 * kChunk);
-                o[0] = r[0]; o[1] = p.y; o[2] = p.x; o[3] = r[-4 * kChunk + 1];
+            for (int cs = 0; cs < 2; ++cs) {
+              const int r3 = wrapk(gz - cs - c30, K3);
+#pragma unroll
+              for (int c2 = 0; c2 < 4; ++c2) {
+                const float* r = phi + phi_index((size_t)r3 * K2 + wrapk(gy - c2, K2), gx, b, P1);
+                float* o = v + (cs * 4 + c2) * 4;
+                if (odd) {   // pairs (gx-1, gx) and (gx-3, gx-2)
+                  const float2 p = *(const float2*)(r - 1), q = *(const float2*)(r - 1 - 2 * kChunk);
+                  o[0] = p.y; o[1] = p.x; o[2] = q.y; o[3] = q.x;
+                } else {     // gx alone, pair (gx-2, gx-1), gx-3 alone
+                  const float2 p = *(const float2*)(r - 2 * kChunk);
+                  o[0] = r[0]; o[1] = p.y; o[2] = p.x; o[3] = r[-4 * kChunk + 1];
+                }
+              }
+            }
+          } else {
+            const int gp = __float_as_int(__shfl_sync(0xffffffffu, rv, src + 14));
+            const int gx = gp & 1023, gy = (gp >> 10) & 1023, gz = gp >> 20;
+            int r1[4];
+#pragma unroll
+            for (int c1 = 0; c1 < 4; ++c1) r1[c1] = (int)phi_index(0, wrapk(gx - c1, K1), b, P1);
+#pragma unroll
+            for (int cs = 0; cs < 2; ++cs) {
+              const int r3 = wrapk(gz - cs - c30, K3);
+#pragma unroll
+              for (int c2 = 0; c2 < 4; ++c2) {
+                const float* rowp = phi + phi_index((size_t)r3 * K2 + wrapk(gy - c2, K2), 0, 0, P1);
+#pragma unroll
+                for (int c1 = 0; c1 < 4; ++c1) v[(cs * 4 + c2) * 4 + c1] = rowp[r1[c1]];
               }
             }
           }
-        } else {
-          const int gp = __float_as_int(__shfl_sync(0xffffffffu, rv, src + 14));
-          const int gx = gp & 1023, gy = (gp >> 10) & 1023, gz = gp >> 20;
-          int r1[4];
-#pragma unroll
-          for (int c1 = 0; c1 < 4; ++c1) r1[c1] = (int)phi_index(0, wrapk(gx - c1, K1), b, P1);
-#pragma unroll
-          for (int cs = 0; cs < 4; ++cs) {
-            const int r3 = wrapk(gz - cs, K3);
-#pragma unroll
-            for (int c2 = 0; c2 < 4; ++c2) {
-              const float* rowp = phi + phi_index((size_t)r3 * K2 + wrapk(gy - c2, K2), 0, 0, P1);
-#pragma unroll
-              for (int c1 = 0; c1 < 4; ++c1) v[(cs * 4 + c2) * 4 + c1] = rowp[r1[c1]];
-            }
-          }
+          // wl[8 + c3] is q w3(c3), formed in FP32 as k_gather<4> forms it; times 1.0f it stays exact
+          accumulate_planes<4, 2>(v, wl, c30, 1.0f, e);
         }
-        // wl[8 + c3] is q w3(c3), formed in FP32 as k_gather<4> forms it; times 1.0f it stays exact
-        accumulate_planes<4, 4>(v, wl, 0, 1.0f, e);
       }
       rv = nxt;
     }
