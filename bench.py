@@ -401,10 +401,12 @@ def main():
     # square 64 planes with direct site sums on the tensor cores run two planes per CTA
     pair = (w.params["ms2max"] == 64 and w.params["ms3max"] == 64 and paths["spectrum_path"] == 2
             and eng.nsite_slt <= 64)
+    plane128 = (w.params["ms2max"] == 128 and w.params["ms3max"] == 128 and paths["spectrum_path"] == 2
+                and eng.nsite_slt <= 64)
     kname = {"gather": "k_gather_rec" if order4 else "k_gather", "bin": "k_bin", "real": "k_real",
              "spread": "k_spread_box", "transpose": "k_transpose_phi",
-             "pme_plane": "k_pme_plane_pair" if pair else "k_pme_plane",
-             "pme_rows": "k_pme_lines" if w.params["ms1max"] <= 64 else "k_pme_rows",
+             "pme_plane": "k_pme_plane_pair" if pair else "k_pme_plane128" if plane128 else "k_pme_plane",
+             "pme_rows": "k_pme_lines" if w.params["ms1max"] <= 64 else "k_pme_lines128",
              "site_tables": "k_site_tables", "influence": "k_influence", "ecorr": "k_ecorr_tma"}
     counters = profile_table("kernel_counters.txt")
     kernels = {}

@@ -1600,7 +1600,7 @@ __global__ void __launch_bounds__(kGatherThreads, NO > 0 ? 4 : 8) k_gather(Frame
 }
 
 // The order-4 gather from per-atom records (k_prepare_solvent) and per-molecule records in
-// cell order (k_mol_records): the same stencil sums as k_gather<4>, in the same order, with
+// cell order (k_mol_groups): the same stencil sums as k_gather<4>, in the same order, with
 // fewer dependent loads.  A warp's first molecule record and the records of its first two
 // atoms are fetched before the wait on the k1 transform (they are frame tables, complete
 // before the chunk chain starts); lanes 0-15 hold one atom's record, lanes 16-31 the next
