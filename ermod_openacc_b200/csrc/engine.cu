@@ -68,6 +68,7 @@ struct ermod_ctx {
   std::vector<int> uvmax, uvsoft;
   DeviceState d;
   int chunk = kChunk, batch = 0, ncell_cap = 0;
+  int longmol = 0;                    // FrameArgs::longmol
   int nhost = 0;                      // atoms of the host aggregate (insposition 2..4)
   int nref = 0;                       // atoms of the RefInfo host (insposition 5, 6)
   bool gauss_init = false;            // Gaussian insertion constants fixed at the first frame
@@ -420,6 +421,9 @@ int32_t ermod_create(ermod_ctx** out, int32_t device, const ermod_params* prm, c
     molq[k] = q;
   }
   ctx->natoms = molbeg[ctx->slvmax];
+  // a single solute in solution meets no copy of itself
+  for (int k = 0; k < ctx->slvmax; ++k)
+    if ((refs || ctx->numslt > 1 || ctx->tagpt[k] != ctx->sltlist[0]) && molbeg[k + 1] - molbeg[k] > kLongMol) ctx->longmol = 1;
   // atoms of the host aggregate (com_aggregate, insertion.F90:587-614): molecules of the hostspec species
   std::vector<int> host_atom;
   std::vector<float> host_mass;
@@ -499,7 +503,7 @@ int32_t ermod_create(ermod_ctx** out, int32_t device, const ermod_params* prm, c
   // PME solve path (spectrum_path): the fused solve where the mesh allows it
   FrameArgs fa{};
   fa.pme = pme; fa.K1 = K1; fa.K2 = K2; fa.K3 = K3; fa.Kh1 = Kh1; fa.nsite = ctx->s; fa.order = order;
-  fa.ljtype_max = ctx->ljtype_max; fa.slvmax = ctx->slvmax; fa.maxdst = ctx->maxdst;
+  fa.ljtype_max = ctx->ljtype_max; fa.slvmax = ctx->slvmax; fa.maxdst = ctx->maxdst; fa.longmol = ctx->longmol;
   if (setup_real_smem(fa) != 0) return bad(ERMOD_ERR_CUDA, "real_smem");
   if (setup_insert_smem(ctx->s) != 0) return bad(ERMOD_ERR_CUDA, "ins_smem");
   const bool fused_ok = pme && fused_supported(fa);
@@ -934,7 +938,7 @@ static int frame_plan(ermod_ctx* ctx, const float* cellin, float wsys, bool use_
   P.screen = p.screen;
   P.ljswitch = p.ljswitch;
   P.bare = p.cltype == ERMOD_EL_COULOMB;
-  a.slvmax = ctx->slvmax; a.natoms = ctx->natoms; a.nsite = ctx->s; a.maxdst = ctx->maxdst;
+  a.slvmax = ctx->slvmax; a.natoms = ctx->natoms; a.nsite = ctx->s; a.maxdst = ctx->maxdst; a.longmol = ctx->longmol;
   a.K1 = K1; a.K2 = K2; a.K3 = K3; a.order = pme ? p.splodr : 1; a.Kh1 = K1 / 2 + 1;
   // Fused solve: planes k1 whose every mode has exp(-pi^2 |k|^2 / screen^2) < kModeCut are not
   // transformed (|k| >= k1 / |a1| in plane k1, a1 the first cell vector).  Their share of any

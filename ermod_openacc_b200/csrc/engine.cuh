@@ -33,6 +33,10 @@ struct MlpLayout {
 };
 
 // Everything the frame kernels read, passed by value.
+// Solvent molecules of more atoms (a protein, a lipid, a polymer) are a serial chain where one lane or
+// warp walks a molecule's atoms: contexts that have one take kernels that allow for it.
+constexpr int kLongMol = 32;
+
 struct FrameArgs {
   CellGeom g;
   PairParams pp;
@@ -46,6 +50,7 @@ struct FrameArgs {
   int use_cells, nc[3];
   float ch[3];                     // cell edge lengths
   float rcut;                      // max(elecut, upljcut): beyond it every pair term is zero
+  int longmol;                     // 1: some solvent molecule has more than kLongMol atoms
 };
 
 // Device-resident state of one context.

@@ -826,6 +826,11 @@ constexpr int kRealYFirst = 64;
 // evaluated 32 a turn, whoever's they are, at the single call of pair_energy, which applies the
 // exact cutoff; each lane last adds up its own energies.
 //
+// A molecule of more than kLongMol atoms (contexts that have one: LONG) is a batch of its own, its atoms
+// dealt to the lanes three at a time; as a lane's work it kept the other 31 waiting.  600 atoms among
+// 512 waters, 160 insertions of 130 sites: 6.96 -> 1.34 ms; 3000 atoms among 4096 waters, 100 of 200
+// sites, the frame 34.8 -> 7.5 ms.  Without one the test for it would cost the ring's frame 3 %.
+//
 // Why: the pair energy (about 200 instructions, erfcf and the exact roots and quotients most of
 // them) bounds the kernel, at 65 % of the issue slots.  A warp that evaluated its lanes' pairs in
 // lockstep spent a pair energy wherever one lane needed it: 15 of 32 lanes were active, and of a
@@ -844,7 +849,7 @@ struct RealWarp {
 // place of hit p: lanes whose runs of up to 16 hits start 16 apart would share two banks
 __device__ __forceinline__ int skew(int p) { return p + (p >> 4); }
 
-template <int LPM>
+template <int LPM, bool LONG>
 __global__ void __launch_bounds__(kRealMaxThreads, 3) k_real(FrameArgs a, int base, int ny,
     const float4* __restrict__ tgt_n, const float4* __restrict__ tgt_c, const int* __restrict__ tgt_mol,
     const int* __restrict__ slt_lj_tab, const int* __restrict__ molbeg, const float4* __restrict__ slvn,
@@ -972,16 +977,33 @@ __global__ void __launch_bounds__(kRealMaxThreads, 3) k_real(FrameArgs a, int ba
       }
       if (qn == 0) break;
       __syncwarp();
-      // the last NB molecules of the queue; lanes past its end take its first entry and store nothing
-      const int nbm = min(NB, qn), mine = lane / LPM;
-      const bool live = mine < nbm;
-      const int4 mr = mrec[q[qn - nbm + (live ? mine : 0)]];
+      // the last NB molecules of the queue; lanes past its end take its last entry and store nothing
+      const int mine = lane / LPM;
+      int nbm = min(NB, qn);
+      bool live = mine < nbm;
+      int4 mr = mrec[q[qn - 1 - (live ? mine : 0)]];
+      // a long molecule is a batch of its own, its atoms shared out to the warp; the batch ends before one
+      const unsigned longs = LONG ? __ballot_sync(0xffffffffu, live && mr.z > kLongMol) : 0u;
+      const bool whole = longs & 1u;
+      if (whole) {
+        nbm = 1;
+        live = true;
+        mr.x = __shfl_sync(0xffffffffu, mr.x, 0);
+        mr.y = __shfl_sync(0xffffffffu, mr.y, 0);
+        mr.z = __shfl_sync(0xffffffffu, mr.z, 0);
+      } else if (longs) {
+        nbm = (__ffs(longs) - 1) / LPM;
+        live = mine < nbm;
+      }
       qn -= nbm;
-      const int njmax = __reduce_max_sync(0xffffffffu, mr.z);
+      const int njmax = __reduce_max_sync(0xffffffffu, live ? mr.z : 0);
+      const int jfirst = whole ? 3 * mine : 0, jstep = whole ? 3 * NB : 3;
+      const bool writes = whole ? lane == 0 : live && sub == 0;
       double* const out = E + (size_t)b * a.slvmax + mr.x;
-      const double before = t > 0 && live && sub == 0 ? *out : 0.0;
+      const double before = t > 0 && writes ? *out : 0.0;
       double acc = 0.0;
-      for (int js0 = 0; js0 < njmax; js0 += 3) {
+      for (int j0 = 0; j0 < njmax; j0 += jstep) {
+        const int js0 = j0 + jfirst;
         float4 xj[3];
         __syncwarp();
 #pragma unroll
@@ -1066,7 +1088,11 @@ __global__ void __launch_bounds__(kRealMaxThreads, 3) k_real(FrameArgs a, int ba
       }
 #pragma unroll
       for (int o = LPM / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      if (live && sub == 0) *out = before + acc;
+      if (whole) {
+#pragma unroll
+        for (int o = LPM; o < 32; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+      }
+      if (writes) *out = before + acc;
       __syncwarp();                 // the next tile's lanes read these sums
     }
   }
@@ -1088,12 +1114,14 @@ size_t real_smem(const FrameArgs& a, int lpm, int threads) {
          sizeof(RealWarp) * (threads / 32);
 }
 
+const void* real_kernel(int lpm, bool longmol) {
+  if (longmol) return lpm == 1 ? (const void*)k_real<1, true> : lpm == 4 ? (const void*)k_real<4, true> : (const void*)k_real<16, true>;
+  return lpm == 1 ? (const void*)k_real<1, false> : lpm == 4 ? (const void*)k_real<4, false> : (const void*)k_real<16, false>;
+}
+
 int setup_real_smem(const FrameArgs& a) {
   const int lpm = real_lpm(a);
-  cudaError_t e = lpm == 1   ? raise_smem_limit(k_real<1>, real_smem(a, 1, kRealMaxThreads))
-                  : lpm == 4 ? raise_smem_limit(k_real<4>, real_smem(a, 4, kRealMaxThreads))
-                             : raise_smem_limit(k_real<16>, real_smem(a, 16, kRealMaxThreads));
-  return e == cudaSuccess ? 0 : -1;
+  return raise_smem_limit_fn(real_kernel(lpm, a.longmol), real_smem(a, lpm, kRealMaxThreads)) == cudaSuccess ? 0 : -1;
 }
 
 // `threads` (a multiple of 32, <= kRealMaxThreads) only changes how the warps share a target's
@@ -1108,12 +1136,16 @@ void launch_real(const FrameArgs& a, const DeviceState& d, int base, int nb, int
   const int ny = std::max(1, std::min((148 * 8 + nb - 1) / nb, (items + threads / 32 - 1) / (threads / 32)));
   const size_t sm = real_smem(a, lpm, threads);
   // launch_k: a graph node of this launch keeps the stream's (lower) priority beside the PME chain
-#define ERM_REAL(L) launch_k(false, dim3(nb, ny), threads, sm, s, k_real<L>, a, base, ny, d.tgt_n, d.tgt_c, d.tgt_mol, \
+#define ERM_REAL(L, G) launch_k(false, dim3(nb, ny), threads, sm, s, k_real<L, G>, a, base, ny, d.tgt_n, d.tgt_c, d.tgt_mol, \
       d.slt_lj, d.molbeg, d.slvn, d.atom_lj, d.ljene, d.ljlensq, (const int4*)d.mrec, (const float4*)d.sanch, \
       (const float4*)d.gsph, d.E)
-  if (lpm == 1) ERM_REAL(1);
-  else if (lpm == 4) ERM_REAL(4);
-  else ERM_REAL(16);
+  if (a.longmol) {
+    if (lpm == 1) ERM_REAL(1, true);
+    else if (lpm == 4) ERM_REAL(4, true);
+    else ERM_REAL(16, true);
+  } else if (lpm == 1) ERM_REAL(1, false);
+  else if (lpm == 4) ERM_REAL(4, false);
+  else ERM_REAL(16, false);
 #undef ERM_REAL
 }
 
