@@ -1631,6 +1631,66 @@ __global__ void __launch_bounds__(kGatherThreads, NO > 0 ? 4 : 8) k_gather(Frame
   }
 }
 
+// One site's share, CS of the four stencil planes at a time: 12 CS loads of a lane in flight beside the
+// sums of the planes before.  Two at a time for the many short molecules of a solvent (60-site chain,
+// 32,768 waters: the frame 33.25 ms against 34.3 with all four; two planes with five to seven CTAs an
+// SM for four: 33.5, 34.1, 35.8).  A long molecule is a chain of sites on one warp, so its loads' latency
+// counts and all four planes go together in contexts that have one (FrameArgs::longmol): gather stage
+// of 1000 insertions with 88 atoms among 3,996 waters 2.35 ms against 2.88.
+template <int CS>
+__device__ __forceinline__ void gather_site(const float* __restrict__ phi, const float (&wl)[12], int off, int flags,
+                                            float rv, int src, int b, int K1, int K2, int K3, int P1, size_t s2,
+                                            size_t s3, double& e) {
+#pragma unroll
+  for (int c30 = 0; c30 < 4; c30 += CS) {
+    float v[CS * 16];
+    if (!(flags & kRecWrap)) {
+      const float* p0 = phi + (size_t)off + 2 * b;
+      if (flags & kRecOdd) gather_rows4<CS, true>(p0, s2, s3, c30, v);
+      else gather_rows4<CS, false>(p0, s2, s3, c30, v);
+    } else if (!(flags & kRecWrapX)) {
+      // only n2 or n3 wraps: each row is contiguous in n1, loaded in pairs as above
+      const int gp = __float_as_int(__shfl_sync(0xffffffffu, rv, src + 14));
+      const int gx = gp & 1023, gy = (gp >> 10) & 1023, gz = gp >> 20;
+      const bool odd = flags & kRecOdd;
+#pragma unroll
+      for (int cs = 0; cs < CS; ++cs) {
+        const int r3 = wrapk(gz - cs - c30, K3);
+#pragma unroll
+        for (int c2 = 0; c2 < 4; ++c2) {
+          const float* r = phi + phi_index((size_t)r3 * K2 + wrapk(gy - c2, K2), gx, b, P1);
+          float* o = v + (cs * 4 + c2) * 4;
+          if (odd) {   // pairs (gx-1, gx) and (gx-3, gx-2)
+            const float2 p = *(const float2*)(r - 1), q = *(const float2*)(r - 1 - 2 * kChunk);
+            o[0] = p.y; o[1] = p.x; o[2] = q.y; o[3] = q.x;
+          } else {     // gx alone, pair (gx-2, gx-1), gx-3 alone
+            const float2 p = *(const float2*)(r - 2 * kChunk);
+            o[0] = r[0]; o[1] = p.y; o[2] = p.x; o[3] = r[-4 * kChunk + 1];
+          }
+        }
+      }
+    } else {
+      const int gp = __float_as_int(__shfl_sync(0xffffffffu, rv, src + 14));
+      const int gx = gp & 1023, gy = (gp >> 10) & 1023, gz = gp >> 20;
+      int r1[4];
+#pragma unroll
+      for (int c1 = 0; c1 < 4; ++c1) r1[c1] = (int)phi_index(0, wrapk(gx - c1, K1), b, P1);
+#pragma unroll
+      for (int cs = 0; cs < CS; ++cs) {
+        const int r3 = wrapk(gz - cs - c30, K3);
+#pragma unroll
+        for (int c2 = 0; c2 < 4; ++c2) {
+          const float* rowp = phi + phi_index((size_t)r3 * K2 + wrapk(gy - c2, K2), 0, 0, P1);
+#pragma unroll
+          for (int c1 = 0; c1 < 4; ++c1) v[(cs * 4 + c2) * 4 + c1] = rowp[r1[c1]];
+        }
+      }
+    }
+    // wl[8 + c3] is q w3(c3), formed in FP32 as k_gather<4> forms it; times 1.0f it stays exact
+    accumulate_planes<4, CS>(v, wl, c30, 1.0f, e);
+  }
+}
+
 // The order-4 gather from per-atom records (k_prepare_solvent) and per-molecule records in
 // cell order (k_mol_groups): the same stencil sums as k_gather<4>, in the same order, with
 // fewer dependent loads.  A warp's first molecule record and the records of its first two
@@ -1641,7 +1701,7 @@ __global__ void __launch_bounds__(kGatherThreads, NO > 0 ? 4 : 8) k_gather(Frame
 // stencils are summed.
 // LK1, LK2 > 0: the mesh's K1 = 2^LK1, K2 = 2^LK2 at compile time, so that every stencil row
 // is the site's base pointer plus a constant offset; 0: taken from FrameArgs.
-template <int LK1, int LK2>
+template <int LK1, int LK2, int CS>
 __global__ void __launch_bounds__(kGatherThreads, 4) k_gather_rec(FrameArgs a, int base, int bb, int nb,
     const int4* __restrict__ mrec, const float* __restrict__ grec, const float* __restrict__ phi,
     const double* __restrict__ tgtq, const int* __restrict__ tgt_mol, double* __restrict__ Etot) {
@@ -1680,57 +1740,7 @@ __global__ void __launch_bounds__(kGatherThreads, 4) k_gather_rec(FrameArgs a, i
         for (int c = 0; c < 12; ++c) wl[c] = __shfl_sync(0xffffffffu, rv, src + c);
         const int off = __float_as_int(__shfl_sync(0xffffffffu, rv, src + 12));
         const int flags = __float_as_int(__shfl_sync(0xffffffffu, rv, src + 13));
-        // two of the four stencil planes at a time: 24 loads of a lane in flight beside the sums of the
-        // two before (all 64 points first: 60-site chain, 32,768 waters, the frame 34.3 against 33.25 ms;
-        // two planes with five to seven CTAs an SM for four: 33.5, 34.1, 35.8)
-#pragma unroll
-        for (int c30 = 0; c30 < 4; c30 += 2) {
-          float v[32];
-          if (!(flags & kRecWrap)) {
-            const float* p0 = phi + (size_t)off + 2 * b;
-            if (flags & kRecOdd) gather_rows4<2, true>(p0, s2, s3, c30, v);
-            else gather_rows4<2, false>(p0, s2, s3, c30, v);
-          } else if (!(flags & kRecWrapX)) {
-            // only n2 or n3 wraps: each row is contiguous in n1, loaded in pairs as above
-            const int gp = __float_as_int(__shfl_sync(0xffffffffu, rv, src + 14));
-            const int gx = gp & 1023, gy = (gp >> 10) & 1023, gz = gp >> 20;
-            const bool odd = flags & kRecOdd;
-#pragma unroll
-            for (int cs = 0; cs < 2; ++cs) {
-              const int r3 = wrapk(gz - cs - c30, K3);
-#pragma unroll
-              for (int c2 = 0; c2 < 4; ++c2) {
-                const float* r = phi + phi_index((size_t)r3 * K2 + wrapk(gy - c2, K2), gx, b, P1);
-                float* o = v + (cs * 4 + c2) * 4;
-                if (odd) {   // pairs (gx-1, gx) and (gx-3, gx-2)
-                  const float2 p = *(const float2*)(r - 1), q = *(const float2*)(r - 1 - 2 * kChunk);
-                  o[0] = p.y; o[1] = p.x; o[2] = q.y; o[3] = q.x;
-                } else {     // gx alone, pair (gx-2, gx-1), gx-3 alone
-                  const float2 p = *(const float2*)(r - 2 * kChunk);
-                  o[0] = r[0]; o[1] = p.y; o[2] = p.x; o[3] = r[-4 * kChunk + 1];
-                }
-              }
-            }
-          } else {
-            const int gp = __float_as_int(__shfl_sync(0xffffffffu, rv, src + 14));
-            const int gx = gp & 1023, gy = (gp >> 10) & 1023, gz = gp >> 20;
-            int r1[4];
-#pragma unroll
-            for (int c1 = 0; c1 < 4; ++c1) r1[c1] = (int)phi_index(0, wrapk(gx - c1, K1), b, P1);
-#pragma unroll
-            for (int cs = 0; cs < 2; ++cs) {
-              const int r3 = wrapk(gz - cs - c30, K3);
-#pragma unroll
-              for (int c2 = 0; c2 < 4; ++c2) {
-                const float* rowp = phi + phi_index((size_t)r3 * K2 + wrapk(gy - c2, K2), 0, 0, P1);
-#pragma unroll
-                for (int c1 = 0; c1 < 4; ++c1) v[(cs * 4 + c2) * 4 + c1] = rowp[r1[c1]];
-              }
-            }
-          }
-          // wl[8 + c3] is q w3(c3), formed in FP32 as k_gather<4> forms it; times 1.0f it stays exact
-          accumulate_planes<4, 2>(v, wl, c30, 1.0f, e);
-        }
+        gather_site<CS>(phi, wl, off, flags, rv, src, b, K1, K2, K3, P1, s2, s3, e);
       }
       rv = nxt;
     }
@@ -1808,19 +1818,21 @@ void launch_gather(const FrameArgs& a, const DeviceState& d, int base, int bb, i
     if (cap == 0) {
       int per_sm = 0, sms = 0;
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gather_rec<0, 0>, kGatherThreads, 0);
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gather_rec<0, 0, 2>, kGatherThreads, 0);
       cap = std::max(1, per_sm * sms);
       if (dev >= 0 && dev < kMaxDevices) resident[dev].store(cap);
     }
     blocks = std::max(1, std::min(blocks, cap));
-#define ERM_GATHER_REC(L1, L2) launch_k(pdl, blocks, kGatherThreads, 0, s, k_gather_rec<L1, L2>, a, base, bb, nb, \
+#define ERM_GATHER_CS(L1, L2, CS) launch_k(pdl, blocks, kGatherThreads, 0, s, k_gather_rec<L1, L2, CS>, a, base, bb, nb, \
       (const int4*)d.mrec, (const float*)d.grec, (const float*)d.phi, (const double*)d.tgtq, (const int*)d.tgt_mol, \
       d.Etot)
+#define ERM_GATHER_REC(L1, L2) (a.longmol ? ERM_GATHER_CS(L1, L2, 4) : ERM_GATHER_CS(L1, L2, 2))
     if (a.K1 == 64 && a.K2 == 64) ERM_GATHER_REC(6, 6);
     else if (a.K1 == 32 && a.K2 == 32) ERM_GATHER_REC(5, 5);
     else if (a.K1 == 128 && a.K2 == 128) ERM_GATHER_REC(7, 7);
     else ERM_GATHER_REC(0, 0);
 #undef ERM_GATHER_REC
+#undef ERM_GATHER_CS
     return;
   }
   if (blocks > 148 * 2048 / kGatherThreads) blocks = 148 * 2048 / kGatherThreads;   // 2048 threads an SM
