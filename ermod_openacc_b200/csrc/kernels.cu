@@ -849,7 +849,7 @@ struct RealWarp {
 // place of hit p: lanes whose runs of up to 16 hits start 16 apart would share two banks
 __device__ __forceinline__ int skew(int p) { return p + (p >> 4); }
 
-template <int LPM, bool LONG>
+template <int LPM, bool LONG, bool TAB>
 __global__ void __launch_bounds__(kRealMaxThreads, 3) k_real(FrameArgs a, int base, int ny,
     const float4* __restrict__ tgt_n, const float4* __restrict__ tgt_c, const int* __restrict__ tgt_mol,
     const int* __restrict__ slt_lj_tab, const int* __restrict__ molbeg, const float4* __restrict__ slvn,
@@ -864,20 +864,22 @@ __global__ void __launch_bounds__(kRealMaxThreads, 3) k_real(FrameArgs a, int ba
   float4* ss = (float4*)rsm_real;              // [s] site positions, charges
   float4* rel = ss + s;                        // [nt TS] positions from the tile's centre, w = LJ type
   float4* tile = rel + nt * TS;                // [nt] centre, radius
-  float* lje = (float*)(tile + nt);
-  float* ljs = lje + ljmax * ljmax;
+  float* sje = (float*)(tile + nt);            // TAB: the LJ tables [ljmax][ljmax]
+  float* sjs = sje + (TAB ? ljmax * ljmax : 0);
+  const float *lje = TAB ? sje : ljene, *ljs = TAB ? sjs : ljlensq;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   // this warp's batch atoms and LJ types, its hits (later their energies), its queue of molecules in reach
-  RealWarp& W = ((RealWarp*)(((uintptr_t)(ljs + ljmax * ljmax) + 15) & ~(uintptr_t)15))[warp];
+  RealWarp& W = ((RealWarp*)(((uintptr_t)(sjs + (TAB ? ljmax * ljmax : 0)) + 15) & ~(uintptr_t)15))[warp];
   float4* satom = W.atom;
   int *slj = W.lj, *slot = W.slot, *q = W.queue;
   const unsigned below = (1u << lane) - 1u;
   const float4* tn = tgt_n + (size_t)cnt * s;
   for (int i = threadIdx.x; i < s; i += blockDim.x) ss[i] = tn[i];
-  for (int i = threadIdx.x; i < ljmax * ljmax; i += blockDim.x) {
-    lje[i] = ljene[i];
-    ljs[i] = ljlensq[i];
-  }
+  if (TAB)
+    for (int i = threadIdx.x; i < ljmax * ljmax; i += blockDim.x) {
+      sje[i] = ljene[i];
+      sjs[i] = ljlensq[i];
+    }
   const int excl = tgt_mol ? tgt_mol[cnt] : -1;
   // soln: solute site LJ types come from the solute molecule's atoms
   const int* site_lj = excl >= 0 ? atom_lj + molbeg[excl] : slt_lj_tab;
@@ -1108,20 +1110,33 @@ int real_lpm(const FrameArgs& a) {
   return lpm;
 }
 
-size_t real_smem(const FrameArgs& a, int lpm, int threads) {
+size_t real_smem(const FrameArgs& a, int lpm, bool tab, int threads) {
   const size_t ts = (size_t)kRealTile * lpm, nt = (a.nsite + ts - 1) / ts;
-  return sizeof(float4) * (a.nsite + nt * ts + nt) + 2 * sizeof(float) * (size_t)a.ljtype_max * a.ljtype_max + 16 +
-         sizeof(RealWarp) * (threads / 32);
+  return sizeof(float4) * (a.nsite + nt * ts + nt) + (tab ? 2 * sizeof(float) * (size_t)a.ljtype_max * a.ljtype_max : 0) +
+         16 + sizeof(RealWarp) * (threads / 32);
 }
 
-const void* real_kernel(int lpm, bool longmol) {
-  if (longmol) return lpm == 1 ? (const void*)k_real<1, true> : lpm == 4 ? (const void*)k_real<4, true> : (const void*)k_real<16, true>;
-  return lpm == 1 ? (const void*)k_real<1, false> : lpm == 4 ? (const void*)k_real<4, false> : (const void*)k_real<16, false>;
+// The LJ tables sit in shared memory up to this many types and are read through L1 above, where they
+// would cost resident CTAs (and, from about 140 types on, not fit).  Frame of 200 insertions of a chain
+// whose every site has its own type, tables in shared memory against L1: 22 types 549 / 558 us, 42
+// types 660 / 657, 62 types 793 / 719, 102 types 1297 / 904.
+constexpr int kRealTabTypes = 32;
+bool real_tab(const FrameArgs& a) { return a.ljtype_max <= kRealTabTypes; }
+
+using RealKernel = void (*)(FrameArgs, int, int, const float4*, const float4*, const int*, const int*, const int*,
+                            const float4*, const int*, const float*, const float*, const int4*, const float4*,
+                            const float4*, double*);
+template <bool LONG, bool TAB>
+RealKernel real_kernel(int lpm) {
+  return lpm == 1 ? k_real<1, LONG, TAB> : lpm == 4 ? k_real<4, LONG, TAB> : k_real<16, LONG, TAB>;
+}
+RealKernel real_kernel(const FrameArgs& a) {
+  const int lpm = real_lpm(a);
+  return !real_tab(a) ? real_kernel<true, false>(lpm) : a.longmol ? real_kernel<true, true>(lpm) : real_kernel<false, true>(lpm);
 }
 
 int setup_real_smem(const FrameArgs& a) {
-  const int lpm = real_lpm(a);
-  return raise_smem_limit_fn(real_kernel(lpm, a.longmol), real_smem(a, lpm, kRealMaxThreads)) == cudaSuccess ? 0 : -1;
+  return raise_smem_limit(real_kernel(a), real_smem(a, real_lpm(a), real_tab(a), kRealMaxThreads)) == cudaSuccess ? 0 : -1;
 }
 
 // `threads` (a multiple of 32, <= kRealMaxThreads) only changes how the warps share a target's
@@ -1134,19 +1149,11 @@ void launch_real(const FrameArgs& a, const DeviceState& d, int base, int nb, int
   if (threads <= 0 || threads > kRealMaxThreads || threads % 32) threads = 256;
   const int lpm = real_lpm(a), items = (a.slvmax + 31) / 32 * lpm;
   const int ny = std::max(1, std::min((148 * 8 + nb - 1) / nb, (items + threads / 32 - 1) / (threads / 32)));
-  const size_t sm = real_smem(a, lpm, threads);
+  const size_t sm = real_smem(a, lpm, real_tab(a), threads);
   // launch_k: a graph node of this launch keeps the stream's (lower) priority beside the PME chain
-#define ERM_REAL(L, G) launch_k(false, dim3(nb, ny), threads, sm, s, k_real<L, G>, a, base, ny, d.tgt_n, d.tgt_c, d.tgt_mol, \
-      d.slt_lj, d.molbeg, d.slvn, d.atom_lj, d.ljene, d.ljlensq, (const int4*)d.mrec, (const float4*)d.sanch, \
-      (const float4*)d.gsph, d.E)
-  if (a.longmol) {
-    if (lpm == 1) ERM_REAL(1, true);
-    else if (lpm == 4) ERM_REAL(4, true);
-    else ERM_REAL(16, true);
-  } else if (lpm == 1) ERM_REAL(1, false);
-  else if (lpm == 4) ERM_REAL(4, false);
-  else ERM_REAL(16, false);
-#undef ERM_REAL
+  launch_k(false, dim3(nb, ny), threads, sm, s, real_kernel(a), a, base, ny, d.tgt_n, d.tgt_c, d.tgt_mol, d.slt_lj,
+           d.molbeg, d.slvn, d.atom_lj, d.ljene, d.ljlensq, (const int4*)d.mrec, (const float4*)d.sanch,
+           (const float4*)d.gsph, d.E);
 }
 
 // ---------------------------------------------------------------------------
