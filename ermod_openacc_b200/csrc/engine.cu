@@ -123,7 +123,7 @@ struct ermod_ctx {
 // With spectrum_path == 0 the fused solve builds the solute spectrum by direct
 // site sums up to this many sites and by plane spreading + forward FFT above:
 // the sums cost s * K2 * K3 per plane, the FFT a fixed ~K2 * K3 * log(K2 K3).
-constexpr size_t kLaneBytes = (size_t)512 << 20;   // largest second lane of the cuFFT path (54^3: 106 MB, 72^3: 251 MB)
+constexpr size_t kLaneBytes = (size_t)512 << 20;   // largest second lane of the cuFFT path (54^3: 122 MB, 72^3: 288 MB, and the plans' work area)
 constexpr int kDirectAutoSites = 16, kDirectAutoSitesTc64 = 32, kDirectAutoSitesTc128 = 64;
 
 enum Stage { kStPrep = 1, kStIns = 2, kStReal = 3, kStSpread = 4, kStR2C = 5, kStInfl = 6, kStC2R = 7,
@@ -244,6 +244,41 @@ size_t frame_zero_bytes(const ermod_ctx* c) { return 64 + sizeof(double) * (size
 // 8-byte words of the accumulators' allocation (DeviceState::edens .. maxuv)
 size_t acc_words(const ermod_ctx* c) {
   return (size_t)c->ermax + std::max(1, c->esmax) + c->numslv + 8 + (size_t)(c->numslv + 1);
+}
+
+// The cuFFT path's second lane (two_lanes), `work` bytes of plan workspace included, in one allocation.
+// An option, so it neither fails a context nor takes more than half of the memory that is free:
+// without it the chunks run on one lane.
+cudaError_t setup_lane(ermod_ctx* c, size_t work) {
+  const size_t K1 = c->p.ms1max, K2 = c->p.ms2max, K3 = c->p.ms3max, Kh1 = K1 / 2 + 1, KK = K1 * K2 * K3, KH = K3 * K2 * Kh1;
+  const size_t C = c->chunk;
+  size_t bytes = 0;
+  auto part = [&](size_t n) { const size_t o = bytes; bytes += (n + 255) / 256 * 256; return o; };
+  const size_t o_spec = part(C * KH * sizeof(float2)), o_phi = part(C * K3 * K2 * 2 * ((K1 + 1) / 2) * sizeof(float));
+  const size_t o_grid = part(C * KK * sizeof(float)), o_phin = part(C * KK * sizeof(float));
+  const size_t o_gacc = part(C * KK * sizeof(long long)), o_box = part(2 * C * sizeof(int4));
+  const size_t o_part = part(C * std::max((size_t)kInflBlocks, Kh1) * sizeof(double)), o_done = part(C * sizeof(unsigned int));
+  const size_t o_work = part(work);
+  size_t free_bytes = 0, total = 0;
+  if (bytes > kLaneBytes || cudaMemGetInfo(&free_bytes, &total) != cudaSuccess || bytes > free_bytes / 2) return cudaSuccess;
+  unsigned char* q = nullptr;
+  if (palloc(c, &q, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    return cudaSuccess;
+  }
+  int lo = 0, hi = 0;
+  cudaError_t e = cudaDeviceGetStreamPriorityRange(&lo, &hi);
+  if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&c->st3, cudaStreamNonBlocking, hi);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_lane, cudaEventDisableTiming);
+  DeviceState& d = c->d1;
+  d.spec = (float2*)(q + o_spec); d.phi = (float*)(q + o_phi); d.grid = (float*)(q + o_grid);
+  d.phin = (float*)(q + o_phin); d.gacc = (long long*)(q + o_gacc); d.boxinfo = (int4*)(q + o_box);
+  d.partial = (double*)(q + o_part); d.done = (unsigned int*)(q + o_done);
+  c->fft_work[1] = q + o_work;
+  if (e == cudaSuccess) e = cudaMemsetAsync(d.grid, 0, sizeof(float) * C * KK, c->st);   // kept zero outside the boxes
+  if (e == cudaSuccess) e = cudaMemsetAsync(d.done, 0, sizeof(unsigned int) * C, c->st);
+  c->two_lanes = e == cudaSuccess;
+  return e;
 }
 
 int set_error(ermod_ctx* c, int code, const char* name) {
@@ -658,6 +693,7 @@ int32_t ermod_create(ermod_ctx** out, int32_t device, const ermod_params* prm, c
     for (int i = 2; i <= 2 * P - 1; ++i) fact *= i;
     for (int l = 0; l < P; ++l) pg.gfb[l] /= fact;
   }
+  size_t lane_work = 0;
   if (pme && ctx->spath == 1) {
     int n[3] = {K3, K2, K1};
     int inR[3] = {K3, K2, K1}, onC[3] = {K3, K2, Kh1};
@@ -674,37 +710,14 @@ int32_t ermod_create(ermod_ctx** out, int32_t device, const ermod_params* prm, c
     CF(cufftMakePlanMany(ctx->c2r, 3, n, inC, 1, (int)KH, onR, 1, (int)KK, CUFFT_C2R, nfft, &work2));
     work = (std::max(work, work2) + 255) / 256 * 256;
     CK(palloc(ctx, (unsigned char**)&ctx->fft_work[0], work));
-    // the second lane: one allocation
-    size_t bytes = 0;
-    auto part = [&](size_t n) { const size_t o = bytes; bytes += (n + 255) / 256 * 256; return o; };
-    const size_t C = ctx->chunk;
-    const size_t o_spec = part(C * KH * sizeof(float2)), o_phi = part(C * K3 * K2 * 2 * ((K1 + 1) / 2) * sizeof(float));
-    const size_t o_grid = part(C * KK * sizeof(float)), o_phin = part(C * KK * sizeof(float));
-    const size_t o_gacc = part(C * KK * sizeof(long long)), o_box = part(2 * C * sizeof(int4));
-    const size_t o_part = part(C * std::max(kInflBlocks, Kh1) * sizeof(double)), o_done = part(C * sizeof(unsigned int));
-    const size_t o_work = part(work);
-    ctx->two_lanes = ctx->batch > ctx->chunk && bytes <= kLaneBytes;
-    if (ctx->two_lanes) {
-      int lo = 0, hi = 0;
-      CK(cudaDeviceGetStreamPriorityRange(&lo, &hi));
-      CK(cudaStreamCreateWithPriority(&ctx->st3, cudaStreamNonBlocking, hi));
-      CK(cudaEventCreateWithFlags(&ctx->ev_lane, cudaEventDisableTiming));
-      unsigned char* q = nullptr;
-      CK(palloc(ctx, &q, bytes));
-      DeviceState& e = ctx->d1;
-      e.spec = (float2*)(q + o_spec); e.phi = (float*)(q + o_phi); e.grid = (float*)(q + o_grid);
-      e.phin = (float*)(q + o_phin); e.gacc = (long long*)(q + o_gacc); e.boxinfo = (int4*)(q + o_box);
-      e.partial = (double*)(q + o_part); e.done = (unsigned int*)(q + o_done);
-      ctx->fft_work[1] = q + o_work;
-      CK(cudaMemsetAsync(e.grid, 0, sizeof(float) * C * KK, st));   // kept zero outside the boxes
-      CK(cudaMemsetAsync(e.done, 0, sizeof(unsigned int) * C, st));
-    }
+    lane_work = work;
   }
   ctx->use_tc = (p.corrcal && ecorr_tc_available() && p.ecorr_path == 0) ? 1 : 0;
   if (ctx->use_tc) {
     ctx->tc_work_bytes = ecorr_tc_workspace(ctx->batch, ctx->ermax);
     CK(palloc(ctx, (unsigned char**)&ctx->tc_work, ctx->tc_work_bytes));
   }
+  if (pme && ctx->spath == 1 && ctx->batch > ctx->chunk) CK(setup_lane(ctx, lane_work));   // behind all that is not optional
   const int rc = ermod_engclear(ctx);
   if (rc != ERMOD_OK) return rc;
   // minuv / maxuv / voffset start values (enginit, engproc.F90:299-303)
