@@ -223,6 +223,11 @@ struct DeviceState {
   float* ins_feat = nullptr; // [maxdst][64] features of each insertion's voxel (training data, on request)
 };
 
+// The process-wide unique number of the allocation that p lies in, 0 where there is none (any more).
+// Buffers kept between calls are checked by it: a host may reset the device (cudaDeviceReset), which
+// frees them and lets the next allocation take their addresses.
+unsigned long long allocation_id(const void* p);
+
 // Copies of pageable host memory through the pinned ring (staging.cu); they return when the bytes
 // have moved.  `q` != 0: the FP64 values divided by it.
 cudaError_t staged_to_host(void* dst, const void* src, size_t bytes, double q, cudaStream_t s);

@@ -40,6 +40,7 @@
 
 namespace erm {
 cudaError_t staged_to_device(void* dst, const void* src, size_t bytes, cudaStream_t s);   // staging.cu
+unsigned long long allocation_id(const void* p);
 }
 
 namespace {
@@ -716,10 +717,11 @@ __global__ void __launch_bounds__(kNT) k_slv_chmpot(SlvArgs a, const double* __r
 // Working memory and stream of a call, kept for the next one: an allocation of this size with its
 // release takes 0.7 ms, now and then several.  At most kKeep per device are kept, none above
 // kKeepBytes; ermod_slvfe_release gives them back.  Taken out under the lock, so calls from
-// several threads have one each.
+// several threads have one each.  A kept one that a device reset has freed, stream and all, is forgotten.
 struct Workspace {
   int device = -1;
   unsigned char* p = nullptr;
+  unsigned long long id = 0;      // p's allocation_id
   size_t bytes = 0;
   cudaStream_t st = nullptr;
 };
@@ -734,9 +736,14 @@ void ws_free(Workspace& w) {
   w = Workspace();
 }
 
+bool ws_lost(const Workspace& w) { return erm::allocation_id(w.p) != w.id; }
+
 bool ws_take(int device, size_t need, Workspace& w) {
   {
     std::lock_guard<std::mutex> lk(g_ws_mu);
+    for (size_t i = 0; i < g_ws.size();)
+      if (ws_lost(g_ws[i])) g_ws.erase(g_ws.begin() + i);
+      else ++i;
     for (size_t i = 0; i < g_ws.size(); ++i)
       if (g_ws[i].device == device && g_ws[i].bytes >= need) {
         w = g_ws[i];
@@ -747,15 +754,17 @@ bool ws_take(int device, size_t need, Workspace& w) {
   w.device = device;
   w.bytes = need;
   if (cudaStreamCreateWithFlags(&w.st, cudaStreamNonBlocking) == cudaSuccess &&
-      cudaMalloc((void**)&w.p, need) == cudaSuccess)
+      cudaMalloc((void**)&w.p, need) == cudaSuccess) {
+    w.id = erm::allocation_id(w.p);
     return true;
+  }
   ws_free(w);
   return false;
 }
 
 // `clean`: the call ended without a CUDA error, its stream is idle
 void ws_give(Workspace& w, bool clean) {
-  if (clean && w.bytes <= kKeepBytes) {
+  if (clean && w.bytes <= kKeepBytes && w.id != 0) {
     std::lock_guard<std::mutex> lk(g_ws_mu);
     int kept = 0;
     for (const Workspace& o : g_ws) kept += o.device == w.device;
@@ -783,6 +792,7 @@ extern "C" const char* ermod_slvfe_last_error(void) { return g_err; }
 extern "C" void ermod_slvfe_release(void) {
   std::lock_guard<std::mutex> lk(g_ws_mu);
   for (Workspace& w : g_ws) {
+    if (ws_lost(w)) continue;
     cudaSetDevice(w.device);
     ws_free(w);
   }

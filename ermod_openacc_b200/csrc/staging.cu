@@ -8,6 +8,7 @@
 // the next slots are in flight, and engstore's division runs on the device, in the kernel that
 // writes the slot.  A division's engstore at 1396 bins, with the small accumulators in one copy: 4.0 ->
 // 0.9 ms.  Where the ring cannot be had, the runtime's own copy does.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -28,6 +29,7 @@ constexpr int kSlots = 12, kWorkers = 4;       // kSlots: a multiple of every wo
 // one ring a process (12 MB), made on first use; a copy holds the lock until its last byte has moved
 std::mutex g_mu;
 unsigned char* g_ring = nullptr;
+unsigned long long g_ring_id = 0;              // its allocation_id: a host's cudaDeviceReset frees the ring
 
 // out = in / q, FP64 quotients as the host forms them
 __global__ void k_divide(size_t n, const double* __restrict__ in, double q, double* __restrict__ out) {
@@ -55,13 +57,18 @@ cudaError_t direct(const Copy& cp) {
 }
 
 bool have_ring() {
+  if (g_ring && allocation_id(g_ring) != g_ring_id) g_ring = nullptr;
   if (g_ring) return true;
   if (cudaHostAlloc((void**)&g_ring, kSlotBytes * kSlots, cudaHostAllocPortable) != cudaSuccess) {
     cudaGetLastError();
     g_ring = nullptr;
     return false;
   }
-  return true;
+  g_ring_id = allocation_id(g_ring);
+  if (g_ring_id != 0) return true;
+  cudaFreeHost(g_ring);
+  g_ring = nullptr;
+  return false;
 }
 
 cudaError_t run(const Copy& cp) {
@@ -159,6 +166,24 @@ cudaError_t run(const Copy& cp) {
 
 }  // namespace
 
+unsigned long long allocation_id(const void* p) {
+  using Query = CUresult (*)(void*, CUpointer_attribute, CUdeviceptr);
+  static std::atomic<Query> query{nullptr};
+  Query f = query.load();
+  if (!f) {
+    void* sym = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPoint("cuPointerGetAttribute", &sym, cudaEnableDefault, &found) != cudaSuccess || !sym) {
+      cudaGetLastError();
+      return 0;
+    }
+    f = (Query)sym;
+    query.store(f);
+  }
+  unsigned long long id = 0;
+  return f(&id, CU_POINTER_ATTRIBUTE_BUFFER_ID, (CUdeviceptr)p) == CUDA_SUCCESS ? id : 0;
+}
+
 cudaError_t staged_to_host(void* dst, const void* src, size_t bytes, double q, cudaStream_t s) {
   return run(Copy{(unsigned char*)dst, (unsigned char*)src, bytes, true, q, s});
 }
@@ -170,6 +195,6 @@ cudaError_t staged_to_device(void* dst, const void* src, size_t bytes, cudaStrea
 
 extern "C" void ermod_staging_release(void) {
   std::lock_guard<std::mutex> lk(erm::g_mu);
-  if (erm::g_ring) cudaFreeHost(erm::g_ring);
+  if (erm::g_ring && erm::allocation_id(erm::g_ring) == erm::g_ring_id) cudaFreeHost(erm::g_ring);
   erm::g_ring = nullptr;
 }

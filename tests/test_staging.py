@@ -1,5 +1,5 @@
 """The pinned ring of large copies (csrc/staging.cu) on the host, with a stand-in for the CUDA calls it makes:
-every length around a slot and the ring, no pinned memory, no events."""
+every length around a slot and the ring, no pinned memory, no events, a device reset between two copies."""
 import os
 import shutil
 import subprocess
@@ -11,6 +11,7 @@ CSRC = os.path.join(ROOT, "ermod_openacc_b200", "csrc")
 # "device" memory is host memory and every copy happens at once; pinned allocations are counted and can fail
 FAKES = r"""
 #pragma once
+#include <cuda.h>
 #include <cuda_runtime.h>
 cudaError_t fk_host_alloc(void**, size_t, unsigned);
 cudaError_t fk_free_host(void*);
@@ -22,6 +23,7 @@ cudaError_t fk_sync(cudaStream_t);
 cudaError_t fk_get_device(int*);
 cudaError_t fk_set_device(int);
 cudaError_t fk_last();
+cudaError_t fk_entry(const char*, void**, unsigned long long, cudaDriverEntryPointQueryResult*);
 #define cudaHostAlloc fk_host_alloc
 #define cudaFreeHost fk_free_host
 #define cudaEventCreateWithFlags fk_event_create
@@ -33,6 +35,7 @@ cudaError_t fk_last();
 #define cudaGetDevice fk_get_device
 #define cudaSetDevice fk_set_device
 #define cudaGetLastError fk_last
+#define cudaGetDriverEntryPoint fk_entry
 """
 
 MAIN = r"""
@@ -51,12 +54,14 @@ static std::map<void*, unsigned long long> live;      // pinned allocations and 
 static unsigned long long next_id = 1;
 static bool fail_pinned = false, fail_events = false;
 static int frees_of_lost = 0, last = 0;
+static void* at = nullptr;                            // a reset lets the next allocation take the same address
 
 cudaError_t fk_host_alloc(void** p, size_t n, unsigned) {
   if (fail_pinned) { last = 2; return cudaErrorMemoryAllocation; }
   std::lock_guard<std::mutex> lk(mu);
-  *p = malloc(n);
-  live[*p] = next_id++;
+  if (!at) at = malloc(n);
+  *p = at;
+  live[at] = next_id++;
   return cudaSuccess;
 }
 cudaError_t fk_free_host(void* p) {
@@ -76,6 +81,18 @@ cudaError_t fk_sync(cudaStream_t) { return cudaSuccess; }
 cudaError_t fk_get_device(int* d) { *d = 0; return cudaSuccess; }
 cudaError_t fk_set_device(int) { return cudaSuccess; }
 cudaError_t fk_last() { const int e = last; last = 0; return (cudaError_t)e; }
+static CUresult fk_attr(void* out, CUpointer_attribute a, CUdeviceptr p) {
+  std::lock_guard<std::mutex> lk(mu);
+  const auto it = live.find((void*)p);
+  if (a != CU_POINTER_ATTRIBUTE_BUFFER_ID || it == live.end()) return CUDA_ERROR_INVALID_VALUE;
+  *(unsigned long long*)out = it->second;
+  return CUDA_SUCCESS;
+}
+cudaError_t fk_entry(const char*, void** f, unsigned long long, cudaDriverEntryPointQueryResult*) {
+  *f = (void*)fk_attr;
+  return cudaSuccess;
+}
+
 static int bad = 0;
 static void check(const char* what, bool ok) {
   if (!ok) { printf("FAILED: %s\n", what); bad = 1; }
@@ -96,6 +113,14 @@ int main() {
                        31 * slot + 24})
     check("ring", copies(bytes, 0.0));
   check("one ring", live.size() == 1);
+  live.clear();                                        // cudaDeviceReset
+  check("after a reset", copies(5 * slot, 0.0) && live.size() == 1);
+  live.clear();
+  live[at] = next_id++;                                // a reset, and the address is another's now
+  ermod_staging_release();
+  check("another's memory is not freed", live.size() == 1);
+  live.clear();
+  check("a ring again", copies(3 * slot, 0.0) && live.size() == 1);
   ermod_staging_release();
   check("released", live.empty() && frees_of_lost == 0);
   ermod_staging_release();
