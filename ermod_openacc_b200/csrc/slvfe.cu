@@ -33,14 +33,13 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
-#include <mutex>
 #include <vector>
 
 #include "../../include/ermod_slvfe.h"
+#include "workspace.cuh"
 
 namespace erm {
 cudaError_t staged_to_device(void* dst, const void* src, size_t bytes, cudaStream_t s);   // staging.cu
-unsigned long long allocation_id(const void* p);
 }
 
 namespace {
@@ -714,68 +713,7 @@ __global__ void __launch_bounds__(kNT) k_slv_chmpot(SlvArgs a, const double* __r
   }
 }
 
-// Working memory and stream of a call, kept for the next one: an allocation of this size with its
-// release takes 0.7 ms, now and then several.  At most kKeep per device are kept, none above
-// kKeepBytes; ermod_slvfe_release gives them back.  Taken out under the lock, so calls from
-// several threads have one each.  A kept one that a device reset has freed, stream and all, is forgotten.
-struct Workspace {
-  int device = -1;
-  unsigned char* p = nullptr;
-  unsigned long long id = 0;      // p's allocation_id
-  size_t bytes = 0;
-  cudaStream_t st = nullptr;
-};
-constexpr size_t kKeepBytes = (size_t)256 << 20;
-constexpr int kKeep = 2;
-std::mutex g_ws_mu;
-std::vector<Workspace> g_ws;
-
-void ws_free(Workspace& w) {
-  if (w.p) cudaFree(w.p);
-  if (w.st) cudaStreamDestroy(w.st);
-  w = Workspace();
-}
-
-bool ws_lost(const Workspace& w) { return erm::allocation_id(w.p) != w.id; }
-
-bool ws_take(int device, size_t need, Workspace& w) {
-  {
-    std::lock_guard<std::mutex> lk(g_ws_mu);
-    for (size_t i = 0; i < g_ws.size();)
-      if (ws_lost(g_ws[i])) g_ws.erase(g_ws.begin() + i);
-      else ++i;
-    for (size_t i = 0; i < g_ws.size(); ++i)
-      if (g_ws[i].device == device && g_ws[i].bytes >= need) {
-        w = g_ws[i];
-        g_ws.erase(g_ws.begin() + i);
-        return true;
-      }
-  }
-  w.device = device;
-  w.bytes = need;
-  if (cudaStreamCreateWithFlags(&w.st, cudaStreamNonBlocking) == cudaSuccess &&
-      cudaMalloc((void**)&w.p, need) == cudaSuccess) {
-    w.id = erm::allocation_id(w.p);
-    return true;
-  }
-  ws_free(w);
-  return false;
-}
-
-// `clean`: the call ended without a CUDA error, its stream is idle
-void ws_give(Workspace& w, bool clean) {
-  if (clean && w.bytes <= kKeepBytes && w.id != 0) {
-    std::lock_guard<std::mutex> lk(g_ws_mu);
-    int kept = 0;
-    for (const Workspace& o : g_ws) kept += o.device == w.device;
-    if (kept < kKeep) {
-      g_ws.push_back(w);
-      w = Workspace();
-      return;
-    }
-  }
-  ws_free(w);
-}
+erm::WorkspaceCache g_ws;         // working memory and stream of a call
 
 int fail(int code, const char* name) {
   g_err = name;
@@ -789,15 +727,7 @@ cudaError_t dalloc(T** p, size_t n) { return cudaMalloc((void**)p, sizeof(T) * (
 
 extern "C" const char* ermod_slvfe_last_error(void) { return g_err; }
 
-extern "C" void ermod_slvfe_release(void) {
-  std::lock_guard<std::mutex> lk(g_ws_mu);
-  for (Workspace& w : g_ws) {
-    if (ws_lost(w)) continue;
-    cudaSetDevice(w.device);
-    ws_free(w);
-  }
-  g_ws.clear();
-}
+extern "C" void ermod_slvfe_release(void) { g_ws.release(); }
 
 extern "C" int32_t ermod_slvfe_delta_mu(int32_t device, int32_t n0, int32_t nsp, int32_t group, int32_t inft,
                                         const double* rho_sln, const double* rho_ref, const double* chi_ref,
@@ -883,8 +813,8 @@ extern "C" int32_t ermod_slvfe_delta_mu_layout(int32_t device, int32_t n0, int32
   const size_t o_spec = take(4 * (size_t)n), o_both = take(4 * (size_t)n);
   // read back in one copy: the results, the check's two maxima, the status, the sweep's verdict
   const size_t o_out = take(8 * (size_t)(nsp + 2) + 8);
-  Workspace ws;
-  bool ok = ws_take(device, used, ws);
+  erm::Workspace ws;
+  bool ok = g_ws.take(device, used, ws);
   if (!ok) return fail(ERMOD_ERR_CUDA, "slv_mem");
   unsigned char* const arena = ws.p;
   const cudaStream_t st = ws.st;
@@ -892,7 +822,7 @@ extern "C" int32_t ermod_slvfe_delta_mu_layout(int32_t device, int32_t n0, int32
     if (sol) cusolverDnDestroy(sol);
     for (void* p : {(void*)d_E, (void*)d_lam, (void*)d_coef, (void*)d_work, (void*)d_info})
       if (p) cudaFree(p);
-    ws_give(ws, ok);
+    g_ws.give(ws, ok);
   };
   auto dp = [&](size_t o) { return (double*)(arena + o); };
   auto ip = [&](size_t o) { return (int*)(arena + o); };

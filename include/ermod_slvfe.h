@@ -86,8 +86,8 @@ int32_t ermod_slvfe_delta_mu_layout(int32_t device, int32_t n, int32_t nsp, int3
                                     const double* aveuv, double slfeng, const ermod_slvfe_opts* opts,
                                     double* chmpt, double* total, int32_t* used_evd);
 
-/* Calls keep up to two working buffers of at most 256 MB per device for the next call; this frees
- * them.  No call may be running. */
+/* Calls keep up to two working buffers of at most 256 MB per device for the next call, the largest
+ * that were used; this frees them and leaves the current device as it is.  No call may be running. */
 void ermod_slvfe_release(void);
 
 /* Name of the last error of ermod_slvfe_delta_mu on this thread. */
