@@ -22,11 +22,13 @@
 
 using namespace erm;
 
+// A reported error is taken off the runtime's thread: the next context's launches are checked by it.
 #define CK(x)                                                   \
   do {                                                          \
     cudaError_t e_ = (x);                                       \
     if (e_ != cudaSuccess) {                                    \
       ctx->err = std::string("cuda: ") + cudaGetErrorString(e_); \
+      cudaGetLastError();                                       \
       return ERMOD_ERR_CUDA;                                    \
     }                                                           \
   } while (0)

@@ -2002,7 +2002,9 @@ cudaError_t raise_smem_limit_fn(const void* kernel, size_t bytes) {
   cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
   if (e != cudaSuccess) return e;
   if ((size_t)fa.maxDynamicSharedSizeBytes >= bytes) return cudaSuccess;
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e != cudaSuccess) cudaGetLastError();   // reported by the caller, not to a later launch's check
+  return e;
 }
 
 // ---------------------------------------------------------------------------
