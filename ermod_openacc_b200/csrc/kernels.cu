@@ -971,7 +971,10 @@ __global__ void __launch_bounds__(kRealMaxThreads, 3) k_real(FrameArgs a, int ba
           float dx = an.x - tc.x, dy = an.y - tc.y, dz = an.z - tc.z;
           min_image(a.g, dx, dy, dz);
           const float lim = a.rcut + tc.w + an.w + margin;
-          in = !(dx * dx + dy * dy + dz * dz > lim * lim) && mrec[m].x != excl;
+          // A sheared cell's image is the nearest one only where that is within half the cell: with a
+          // larger reach a molecule whose image is out of it may have a site whose own image is not.
+          const bool far = dx * dx + dy * dy + dz * dz > lim * lim && (metric || lim < halfbox);
+          in = !far && mrec[m].x != excl;
         }
         const unsigned bal = __ballot_sync(0xffffffffu, in);
         if (in) q[qn + __popc(bal & below)] = m;
