@@ -529,11 +529,16 @@ int32_t ermod_create(ermod_ctx** out, int32_t device, const ermod_params* prm, c
   d.insw_in = (float*)((unsigned char*)d.frame_i + kInHead);
   d.posraw = d.insw_in + MD;
   d.ins_conf = d.posraw + 3 * NA;
-  CK(palloc(ctx, &d.slvn, NA)); CK(palloc(ctx, &d.spl, NA * 3 * order)); CK(palloc(ctx, &d.grd, NA));
-  if (pme && gather_rec_ok(order, K1, K2, K3)) CK(palloc(ctx, &d.grec, NA * kRecWords));
+  CK(palloc(ctx, &d.slvn, NA));
+  if (pme && gather_rec_ok(order, K1, K2, K3)) {
+    CK(palloc(ctx, &d.grec, NA * kRecWords));
+  } else if (pme) {
+    CK(palloc(ctx, &d.spl, NA * 3 * order));
+    CK(palloc(ctx, &d.grd, NA));
+  }
   CK(palloc(ctx, &d.mrec, SM)); CK(palloc(ctx, &d.sanch, SM)); CK(palloc(ctx, &d.gsph, (SM + 31) / 32));
   CK(palloc(ctx, &d.anchor, SM)); CK(palloc(ctx, &d.cellof, SM)); CK(palloc(ctx, &d.cellcount, ctx->ncell_cap));
-  CK(palloc(ctx, &d.cellstart, ctx->ncell_cap + 1)); CK(palloc(ctx, &d.molsorted, SM));
+  CK(palloc(ctx, &d.molsorted, SM));
   CK(palloc(ctx, &d.tgt_raw, MD * S)); CK(palloc(ctx, &d.tgt_n, MD * S)); CK(palloc(ctx, &d.tgt_c, MD)); CK(palloc(ctx, &d.tgt_mol, MD));
   CK(palloc(ctx, &d.selfreal, MD)); CK(palloc(ctx, &d.u0, MD)); CK(palloc(ctx, &d.w, MD));
   const size_t KK = (size_t)K1 * K2 * K3, KH = (size_t)K3 * K2 * Kh1;

@@ -146,7 +146,6 @@ struct DeviceState {
   float4* anchor = nullptr;  // [slvmax] first-site position, w = molecule extent
   int* cellof = nullptr;     // [slvmax]
   int* cellcount = nullptr;  // [ncell_cap]
-  int* cellstart = nullptr;  // [ncell_cap+1]
   int* molsorted = nullptr;  // [slvmax]
   // per frame: targets (insertions or soln solutes)
   float* ins_conf = nullptr; // [3*s*maxdst] staging of caller conformations
@@ -170,7 +169,7 @@ struct DeviceState {
                              // P1 = ceil(K1 / 2); see phi_index
   float* engfac = nullptr;   // [K3*K2*Kh1]
   float* engfacT = nullptr;  // [Kh1*K3*K2] influence function, k1-major (fused PME solve)
-  float2* fft_tw = nullptr;  // [K1+K2+K3+K1/2] FP32 twiddle tables of the fused PME solve
+  float2* fft_tw = nullptr;  // [K1+K2+K3] FP32 twiddle tables of the fused PME solve
   double2* fft_twd = nullptr;// [K1+K2+K3] FP64 twiddle tables (stencil transforms)
   float2* sitetab = nullptr; // [batch*s*(Kh1 [+K2+K3])] per (target, site) stencil transforms of a batch
   float* sitestn = nullptr;  // [batch*s*(2+2*kMaxOrder)] per (target, site) stencils (plane spreading)

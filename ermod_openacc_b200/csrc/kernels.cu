@@ -144,7 +144,7 @@ __global__ void k_anchor(FrameArgs a, const int* __restrict__ molbeg, const floa
 }
 
 // exclusive scan of the cell counts in one block; leaves cellcount = start (fill cursor)
-__global__ void k_cell_scan(int ncell, int* __restrict__ cellcount, int* __restrict__ cellstart) {
+__global__ void k_cell_scan(int ncell, int* __restrict__ cellcount) {
   __shared__ int part[1024];
   const int t = threadIdx.x, nt = blockDim.x;
   const int per = (ncell + nt - 1) / nt;
@@ -162,11 +162,9 @@ __global__ void k_cell_scan(int ncell, int* __restrict__ cellcount, int* __restr
   int run = part[t] - s;
   for (int i = lo; i < hi; ++i) {
     const int c = cellcount[i];
-    cellstart[i] = run;
     cellcount[i] = run;
     run += c;
   }
-  if (t == nt - 1) cellstart[ncell] = part[nt - 1];
 }
 
 __global__ void k_cell_fill(int slvmax, const int* __restrict__ cellof, int* __restrict__ cursor,
@@ -226,7 +224,7 @@ void launch_cells(const FrameArgs& a, const DeviceState& d, int ncell, cudaStrea
   if (a.use_cells) cudaMemsetAsync(d.cellcount, 0, sizeof(int) * ncell, s);
   k_anchor<<<(a.slvmax + 255) / 256, 256, 0, s>>>(a, d.molbeg, d.slvn, d.anchor, d.cellof, d.cellcount);
   if (a.use_cells) {
-    k_cell_scan<<<1, 1024, 0, s>>>(ncell, d.cellcount, d.cellstart);
+    k_cell_scan<<<1, 1024, 0, s>>>(ncell, d.cellcount);
     k_cell_fill<<<(a.slvmax + 255) / 256, 256, 0, s>>>(a.slvmax, d.cellof, d.cellcount, d.molsorted);
   } else {
     k_iota<<<(a.slvmax + 255) / 256, 256, 0, s>>>(a.slvmax, d.molsorted);
@@ -2016,8 +2014,8 @@ cudaError_t raise_smem_limit_fn(const void* kernel, size_t bytes) {
 // One CTA for a batch: the offset, every target's weight engnmfc (engproc.F90:883-903, volcorrect
 // :1022-1038) and the batch's scalar accumulators, summed in a fixed order (engproc.F90:905-915,
 // 939-941): engnorm, engsmpl, avslf, the self-energy histogram, slnuv (soln) and the self-energy
-// min / max.  At most 4096 targets, four a thread.  One target: 3.5 us, where a launch each for offset,
-// weights and sums took 8 with their gaps.
+// min / max.  A batch has 4096 targets, four a thread, unless the caller asks for more.  One target: 3.5
+// us, where a launch each for offset, weights and sums took 8 with their gaps.
 constexpr int kSumThreads = 1024;
 
 __global__ void __launch_bounds__(kSumThreads) k_weights(WeightArgs wa, int base, int n, const int* __restrict__ skip,

@@ -1304,17 +1304,16 @@ size_t fused_sitetab_elems(const FrameArgs& a, int batch, bool direct) {
 size_t fused_sitestn_elems(const FrameArgs& a, int batch) { return (size_t)batch * a.nsite * kStn; }
 
 void fused_twiddles(int K1, int K2, int K3, std::vector<float2>& tw, std::vector<double2>& twd) {
-  // tw:  [K1 | K2 | K3 | K1/2] tables of exp(-2 pi i m / N), FP64 rounded to FP32
-  // twd: [K1 | K2 | K3] the same in FP64
+  // [K1 | K2 | K3] tables of exp(-2 pi i m / N), FP64 rounded to FP32 and in FP64
   tw.clear();
   twd.clear();
-  const int Ns[4] = {K1, K2, K3, K1 / 2};
-  for (int t = 0; t < 4; ++t)
+  const int Ns[3] = {K1, K2, K3};
+  for (int t = 0; t < 3; ++t)
     for (int m = 0; m < Ns[t]; ++m) {
       const double ang = 2.0 * kPi * (double)m / (double)Ns[t];
       const double c = std::cos(ang), sn = -std::sin(ang);
       tw.push_back(make_float2((float)c, (float)sn));
-      if (t < 3) twd.push_back(make_double2(c, sn));
+      twd.push_back(make_double2(c, sn));
     }
 }
 
