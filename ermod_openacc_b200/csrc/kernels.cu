@@ -808,8 +808,9 @@ void launch_selfreal(const FrameArgs& a, const DeviceState& d, int first, int co
 // ---------------------------------------------------------------------------
 constexpr int kRealMaxThreads = 256;
 constexpr int kRealTile = 16;      // solute sites a lane tests at a time
-// Energies keep the bits that the library's results have had: the squared distance is rounded as
-// (y^2 + x^2) + z^2 for solutes of up to this many sites and as (x^2 + y^2) + z^2 above.
+// The squared distance is rounded as (y^2 + x^2) + z^2 for solutes of up to this many sites and as
+// (x^2 + y^2) + z^2 above, for no reason but that every FP32 pair energy then has the bits that earlier
+// versions gave it, and no count near a bin's edge moves.
 constexpr int kRealYFirst = 64;
 
 // A molecule is taken by LPM lanes, its sites dealt out to them in turn; each lane adds its pair
@@ -830,10 +831,10 @@ constexpr int kRealYFirst = 64;
 // sites, the frame 34.8 -> 7.5 ms.  Without one the test for it would cost the ring's frame 3 %.
 //
 // Why: the pair energy (about 200 instructions, erfcf and the exact roots and quotients most of
-// them) bounds the kernel, at 65 % of the issue slots.  A warp that evaluated its lanes' pairs in
+// them) bounds the kernel, at 60 % of the issue slots with 2000 insertions of the ring.  A warp that evaluated its lanes' pairs in
 // lockstep spent a pair energy wherever one lane needed it: 15 of 32 lanes were active, and of a
-// chain's sites 94 % lay beyond the cutoff of the molecules in reach.  Listing the hits keeps 31
-// lanes active; the spheres per tile leave out most of what a long chain does not reach.
+// chain's sites 94 % lay beyond the cutoff of the molecules in reach.  Listing the hits keeps 27
+// lanes active over the whole kernel; the spheres per tile leave out most of what a long chain does not reach.
 // Measured before and with it, real-space stage of one frame: 12-site ring, 2000 insertions into
 // 4096 waters 0.43 -> 0.29 ms; 60-site chain, 2048 into 32,768 waters 7.1 -> 2.1 ms; 200 sites,
 // 4000 into 4096 waters 24.2 -> 8.8 ms; one 60-site solute in solution, 4096 waters (one CTA

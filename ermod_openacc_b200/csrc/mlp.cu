@@ -42,7 +42,7 @@ namespace {
 // and the bias sums 0.30 ms on one warp each.  Split over the samples, 128 CTAs fill the chip once
 // and the intermediates d1..d3 stay in shared memory: k_bwd 34 us, k_bwd_sum 7 us, the call 213 us.
 // The products are FP32 FMAs (0.74 GFLOP a batch of 4096, about 10 us of the chip's FMA pipes), one
-// CTA an SM by its 179 KB; what is left is the staging and the shared-memory reads of the products.
+// CTA an SM by its 168 KB; what is left is the staging and the shared-memory reads of the products.
 // The partial rows (21 MB) stay in L2.
 constexpr int kBwdRows = 32, kBwdThreads = 256;
 constexpr int kBwdParts = 296;     // rows of `part` at most (two waves of one CTA an SM): larger batches loop

@@ -344,7 +344,8 @@ __device__ __forceinline__ uint32_t site_mma64(const float2* __restrict__ tab, s
     for (int u = 0; u < NI; ++u) {
       const int t = ta + 2 * u, v = tb + 4 * (u >> 1), k3 = qb + 32 * (u & 1);
       if (t < 4 * nks) {
-        // q B1(k1) B2(k2 = qa); zero when off.  The roundings are fixed here, one form for each plane.
+        // q B1(k1) B2(k2 = qa); zero when off.  The roundings are fixed here, one form for each half (a
+        // plane's last bits depend on its half), as earlier versions had them.
         const float2 d = make_float2(__fmaf_rn(cA[u].x, b2[u].x, -__fmul_rn(cA[u].y, b2[u].y)),
                                      __fmaf_rn(cA[u].y, b2[u].x, __fmul_rn(cA[u].x, b2[u].y)));
         put_split2(ahi, alo, qa, 2 * t, d.x, d.y);
@@ -818,7 +819,7 @@ __global__ void __launch_bounds__(2 << LK, 3) k_pme_plane_pair(FrameArgs a, int 
 // The plane crosses shared memory eight times where the stage by stage transform took fourteen.
 // Measured on the 60-site chain, 2048 insertions into 32,768 waters (52 planes, four tiles of sites):
 // the plane stage 21.5 -> 16.4 ms a frame, the frame 40.1 -> 35.1 ms.  With one CTA an SM (200 KB), its
-// phases follow one another: issue slots 46 % busy, shared memory 48 %, tensor pipe 15 %.
+// phases follow one another: issue slots 45 % busy, L1 and shared memory 49 %, tensor pipe 15 %.
 // ---------------------------------------------------------------------------
 constexpr int kRowPitch128 = 152;
 

@@ -213,6 +213,8 @@ int32_t ermod_enginit_mesh(const ermod_hist* hist, int32_t numslv,
  * the caller's arrays may be freed afterwards.  Replaces the one-time
  * setup done by enginit (engproc.F90:36-319), recpcal_init
  * (recpcal.F90:40-95) and instslt('init') (insertion.F90:48-62).
+ * A solute has at most 1024 sites (ERMOD_ERR_OVERFLOW, "ins_siz"); solvent
+ * molecules and LJ types are limited by the device's memory only.
  */
 int32_t ermod_create(ermod_ctx** out, int32_t device, const ermod_params* params,
                      const ermod_topology* topo, const ermod_mesh* mesh);
@@ -252,6 +254,14 @@ int32_t ermod_engclear(ermod_ctx* ctx);
  *                       structure weight (insertion.F90:541-542).
  *   flceng              soln only: [numslv*numslt] per-solute energy sums
  *                       (engproc.F90:918,932), or NULL.
+ *
+ * The same calls on contexts of the same parameters give the same bits (but
+ * flceng and slnuv with several solvent species, whose FP64 sums take the
+ * order of arrival).  The order of the FP64 sums over an energy's terms, and
+ * the FP32 rounding of its mesh terms on some meshes, depend on the number of
+ * targets and on a target's place in its chunk of 32: contexts of other
+ * maxins, or ranks with other shares of the insertions, agree to rounding and
+ * not to the last bit.
  */
 int32_t ermod_engconst(ermod_ctx* ctx, int32_t stnum, const float* sitepos,
                        const float* cell, float stat_weight_system,
