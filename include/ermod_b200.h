@@ -333,7 +333,8 @@ int32_t ermod_get_paths(const ermod_ctx* ctx, int32_t* spectrum_path, int32_t* e
 
 /* Large results and inputs (the correlation matrix of engstore, fetch_accum and slvfe) pass
  * through one 12 MB ring of pinned memory a process, kept between calls; this frees it.  No
- * such call may be running. */
+ * such call may be running.  Where the ring cannot be had the copies go without it, and after
+ * a cudaDeviceReset it is made anew. */
 void ermod_staging_release(void);
 
 /* Kernel launches of this library since the context was created, cuFFT's

@@ -41,7 +41,10 @@ def test_two_lanes_give_the_bits_of_one(engine_lib, maxins, batch, mesh, order):
 def test_no_memory_for_a_second_lane(engine_lib):
     """With room for one lane only (here 40 MB less than an engine with both uses, of which the second
     lane is 86 MB and more), the engine is made and gives the same energies."""
+    import gc
+
     import torch
+    gc.collect()                                    # engines of earlier tests give their memory back now
     w = S.make_workload(2, small=True, maxins=97)
     prm = dict(w.params, keep_uvengy=1, corrcal=0, ms1max=48, ms2max=48, ms3max=48)
     eng = Engine(prm, w.topo, w.hist)               # loads what a first engine loads
